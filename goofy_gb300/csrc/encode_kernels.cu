@@ -4,11 +4,14 @@
 // compressETC1, GoofyTC/goofy_tc.h:1497-1557: block rows x 16-pixel strips,
 // 4 blocks per goofySimdEncode call) with a grid over 4x4 blocks.
 //
-// Mapping: one warp owns a segment of 32*BPT consecutive blocks of one block
-// row; lane l encodes blocks l, l+32, ..., l+32*(BPT-1) of the segment.  For
-// each of the 4 pixel rows a warp-wide 128-bit load instruction therefore
-// reads 512 contiguous bytes (every 32-byte sector fully used), and each
-// 8-byte block store of the warp writes 256 contiguous bytes.  Source rows are
+// Mapping: one warp owns a segment of 32*BPT consecutive blocks of the image
+// in row-major order; lane l encodes blocks l, l+32, ..., l+32*(BPT-1) of the
+// segment.  For each of the 4 pixel rows a warp-wide 128-bit load instruction
+// therefore reads 512 contiguous bytes (every 32-byte sector fully used; two
+// runs where the segment crosses into the next block row), and each 8-byte
+// block store of the warp writes 256 contiguous bytes.  Segments that ended
+// with their block row left most lanes idle on narrow images (120x8000 ETC1s:
+// 7.0 us then, 2.0 us so).  Source rows are
 // read once (L1 no-allocate) and blocks are written with streaming stores:
 // the kernel moves 4 B/px in and 0.5 B/px out and is meant to sit on the HBM
 // roofline.  Launched with programmatic dependent launch (pdl.cuh): CTAs may
@@ -16,6 +19,7 @@
 // their first load.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <atomic>
 
 #include "block_codec.cuh"
@@ -31,43 +35,41 @@ __device__ __forceinline__ void load_block(const uint8_t* p, size_t stride, uint
     load_block_rows(p, stride, ACCESS == SrcAccess::kVec16, w);
 }
 
-struct Segment {
-    uint32_t by, bx0;  // block row, first block of this lane
-};
-
+// Loads this lane's blocks of segment `seg`: blocks b0, b0 + 32, ... of the
+// image in row-major order (b0 returned), so a segment runs on from one block
+// row into the next and only the image's last one is short.
 template <int BPT, SrcAccess ACCESS>
-__device__ __forceinline__ Segment load_segment(const uint8_t* __restrict__ src, size_t stride, uint32_t bw,
-                                                uint32_t seg, uint32_t segs_per_row, uint32_t seg_magic,
-                                                uint32_t lane, uint32_t (&w)[BPT][16])
+__device__ __forceinline__ uint32_t load_segment(const uint8_t* __restrict__ src, size_t stride, uint32_t bw,
+                                                 uint32_t bw_magic, uint32_t total, uint32_t seg, uint32_t lane,
+                                                 uint32_t (&w)[BPT][16])
 {
-    uint32_t sx;
-    Segment sg;
-    sg.by = div_magic(seg, segs_per_row, seg_magic, sx);
-    sg.bx0 = sx * (32u * BPT) + lane;
-    const uint8_t* row = src + (size_t)sg.by * 4u * stride;
+    const uint32_t b0 = seg * (32u * BPT) + lane;
 #pragma unroll
     for (int j = 0; j < BPT; ++j) {
-        const uint32_t bx = sg.bx0 + 32u * j;
-        if (bx < bw) load_block<ACCESS>(row + 16u * (size_t)bx, stride, w[j]);
+        const uint32_t b = b0 + 32u * j;
+        if (b < total) {
+            uint32_t bx;
+            const uint32_t by = div_magic(b, bw, bw_magic, bx);
+            load_block<ACCESS>(src + (size_t)by * 4u * stride + 16u * (size_t)bx, stride, w[j]);
+        }
     }
-    return sg;
+    return b0;
 }
 
 template <int CODEC, int BPT>
-__device__ __forceinline__ void encode_segment(uint8_t* __restrict__ dst, uint8_t* __restrict__ dst2, uint32_t bw,
-                                               Segment sg, const uint32_t (&w)[BPT][16], const uint8_t* ctrl_lut)
+__device__ __forceinline__ void encode_segment(uint8_t* __restrict__ dst, uint8_t* __restrict__ dst2, uint32_t total,
+                                               uint32_t b0, const uint32_t (&w)[BPT][16], const uint8_t* ctrl_lut)
 {
-    const size_t row = (size_t)sg.by * bw * 8u;
 #pragma unroll
     for (int j = 0; j < BPT; ++j) {
-        const uint32_t bx = sg.bx0 + 32u * j;
-        if (bx < bw) {
+        const uint32_t b = b0 + 32u * j;
+        if (b < total) {
             if constexpr (CODEC == kBoth) {
                 const uint4 e = encode_both(w[j], ctrl_lut);
-                st_stream8(dst + row + 8u * (size_t)bx, make_uint2(e.x, e.y));
-                st_stream8(dst2 + row + 8u * (size_t)bx, make_uint2(e.z, e.w));
+                st_stream8(dst + 8u * (size_t)b, make_uint2(e.x, e.y));
+                st_stream8(dst2 + 8u * (size_t)b, make_uint2(e.z, e.w));
             } else {
-                st_stream8(dst + row + 8u * (size_t)bx, encode_block<CODEC>(w[j], ctrl_lut));
+                st_stream8(dst + 8u * (size_t)b, encode_block<CODEC>(w[j], ctrl_lut));
             }
         }
     }
@@ -80,8 +82,7 @@ __device__ __forceinline__ void encode_segment(uint8_t* __restrict__ dst, uint8_
 template <int CODEC, int BPT, SrcAccess ACCESS>
 __global__ void __launch_bounds__(512) encode_image_kernel(const uint8_t* __restrict__ src, size_t stride,
                                                            uint8_t* __restrict__ dst, uint8_t* __restrict__ dst2,
-                                                           uint32_t bw, uint32_t total_segs, uint32_t segs_per_row,
-                                                           uint32_t seg_magic)
+                                                           uint32_t bw, uint32_t bw_magic, uint32_t total)
 {
     pdl_launch_dependents();
     __shared__ uint8_t ctrl_lut[128];
@@ -90,18 +91,17 @@ __global__ void __launch_bounds__(512) encode_image_kernel(const uint8_t* __rest
         __syncthreads();
     }
     const uint32_t seg = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (seg >= total_segs) return;
+    if (seg * (32u * BPT) >= total) return;
     pdl_wait();
     uint32_t w[BPT][16];
-    const Segment sg = load_segment<BPT, ACCESS>(src, stride, bw, seg, segs_per_row, seg_magic, threadIdx.x & 31u, w);
-    encode_segment<CODEC, BPT>(dst, dst2, bw, sg, w, ctrl_lut);
+    const uint32_t b0 = load_segment<BPT, ACCESS>(src, stride, bw, bw_magic, total, seg, threadIdx.x & 31u, w);
+    encode_segment<CODEC, BPT>(dst, dst2, total, b0, w, ctrl_lut);
 }
 
 template <int CODEC, int BPT, SrcAccess ACCESS>
 __global__ void __launch_bounds__(512) encode_image_persistent(const uint8_t* __restrict__ src, size_t stride,
                                                                uint8_t* __restrict__ dst, uint32_t bw,
-                                                               uint32_t total_segs, uint32_t segs_per_row,
-                                                               uint32_t seg_magic)
+                                                               uint32_t bw_magic, uint32_t total)
 {
     pdl_launch_dependents();
     __shared__ uint8_t ctrl_lut[128];
@@ -112,19 +112,19 @@ __global__ void __launch_bounds__(512) encode_image_persistent(const uint8_t* __
     pdl_wait();
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t warp_stride = gridDim.x * (blockDim.x >> 5);
+    const uint32_t segs = (total + 32u * BPT - 1u) / (32u * BPT);
     uint32_t seg = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    uint32_t a[BPT][16], b[BPT][16];
-    Segment sa{}, sb{};
-    if (seg < total_segs) sa = load_segment<BPT, ACCESS>(src, stride, bw, seg, segs_per_row, seg_magic, lane, a);
-    while (seg < total_segs) {
+    uint32_t a[BPT][16], b[BPT][16], ba = 0, bb = 0;
+    if (seg < segs) ba = load_segment<BPT, ACCESS>(src, stride, bw, bw_magic, total, seg, lane, a);
+    while (seg < segs) {
         uint32_t next = seg + warp_stride;
-        if (next < total_segs) sb = load_segment<BPT, ACCESS>(src, stride, bw, next, segs_per_row, seg_magic, lane, b);
-        encode_segment<CODEC, BPT>(dst, nullptr, bw, sa, a, ctrl_lut);
+        if (next < segs) bb = load_segment<BPT, ACCESS>(src, stride, bw, bw_magic, total, next, lane, b);
+        encode_segment<CODEC, BPT>(dst, nullptr, total, ba, a, ctrl_lut);
         seg = next;
-        if (seg >= total_segs) break;
+        if (seg >= segs) break;
         next = seg + warp_stride;
-        if (next < total_segs) sa = load_segment<BPT, ACCESS>(src, stride, bw, next, segs_per_row, seg_magic, lane, a);
-        encode_segment<CODEC, BPT>(dst, nullptr, bw, sb, b, ctrl_lut);
+        if (next < segs) ba = load_segment<BPT, ACCESS>(src, stride, bw, bw_magic, total, next, lane, a);
+        encode_segment<CODEC, BPT>(dst, nullptr, total, bb, b, ctrl_lut);
         seg = next;
     }
 }
@@ -171,22 +171,19 @@ static cudaError_t launch_t(const uint8_t* src, size_t stride, uint8_t* dst, uin
     constexpr bool kHasPersistent = BPT <= 2 && CODEC != kBoth;
     prefer_shared(encode_image_kernel<CODEC, BPT, ACCESS>, 0);
     if constexpr (kHasPersistent) prefer_shared(encode_image_persistent<CODEC, BPT, ACCESS>, 1);
-    const uint32_t segs = (bw + 32u * BPT - 1) / (32u * BPT);
-    const uint64_t total = (uint64_t)segs * bh;
-    if (total > 0x7fffffffull) return cudaErrorInvalidValue;
-    const uint32_t wpc = threads / 32u;
-    uint64_t ctas = (total + wpc - 1) / wpc;
-    const uint32_t magic = 0xffffffffu / segs;
+    const uint32_t total = bw * bh, magic = 0xffffffffu / bw;
+    const uint32_t per_cta = threads * BPT;
+    uint64_t ctas = ((uint64_t)total + per_cta - 1) / per_cta;
     if constexpr (kHasPersistent) {
         if (persistent) {
             const uint64_t resident = (uint64_t)resident_ctas<CODEC, BPT, ACCESS>(threads);
             if (ctas > resident) ctas = resident;
             return launch_pdl(encode_image_persistent<CODEC, BPT, ACCESS>, dim3((unsigned)ctas), dim3(threads), 0,
-                              stream, src, stride, dst, bw, (uint32_t)total, segs, magic);
+                              stream, src, stride, dst, bw, magic, total);
         }
     }
     return launch_pdl(encode_image_kernel<CODEC, BPT, ACCESS>, dim3((unsigned)ctas), dim3(threads), 0, stream, src,
-                      stride, dst, dst2, bw, (uint32_t)total, segs, magic);
+                      stride, dst, dst2, bw, magic, total);
 }
 
 template <int CODEC, SrcAccess ACCESS>
@@ -219,10 +216,40 @@ cudaError_t launch_image(int codec, const uint8_t* src, size_t stride, uint8_t* 
     if (codec != kBC1 && codec != kETC1S && (codec != kBoth || !dst2)) return cudaErrorInvalidValue;
     const uint32_t bw = width / 4, bh = height / 4;
     if (bw == 0 || bh == 0) return cudaSuccess;
+    constexpr uint64_t kMostBlocks = 1u << 30;  // a launch numbers its blocks in 32 bits
+    if ((uint64_t)bw * bh > kMostBlocks) {      // in bands of block rows (a row has fewer: its stride is 32 bits)
+        const uint32_t band = (uint32_t)(kMostBlocks / bw);
+        for (uint32_t y = 0; y < bh; y += std::min(band, bh - y)) {
+            const size_t out = (size_t)y * bw * 8u;
+            const cudaError_t e = launch_image(codec, src + (size_t)y * 4u * stride, stride, dst + out, width,
+                                               4u * std::min(band, bh - y), tile, access, stream,
+                                               dst2 ? dst2 + out : nullptr);
+            if (e != cudaSuccess) return e;
+        }
+        return cudaSuccess;
+    }
     if (tile.persistent == 2) {
-        if (access == SrcAccess::kVec16)
+        // Launches back to back over inputs of 400 MB in all (us), BC1 / ETC1s / both:
+        //                            grid 128x1           bulk copy 128x1      bulk copy 512x2
+        //   256^2     (4096 blocks)   1.6 / 1.8 / 1.7      1.6 / 1.7 / 1.7      4.1 / 4.4 / 4.7
+        //   512^2     (16384)         1.7 / 2.0 / 2.5      2.2 / 2.3 / 2.8      3.1 / 3.5 / 3.8
+        //   1024^2    (65536)         3.4 / 2.9 / 3.5      2.7 / 2.5 / 3.1      2.8 / 3.2 / 3.4
+        //   2048^2    (262144)        4.9 / 5.5 / 5.9      4.6 / 4.9 / 5.7      4.8 / 5.5 / 6.1
+        //   3840x2160 (518400)        7.7 / 9.0 / 9.6      6.7 / 7.3 / 8.4      7.1 / 8.1 / 9.0
+        //   3600x3400 (765000)       11.2 / 12.4 / 13.2   10.0 / 10.7 / 12.8    9.3 / 10.4 / 12.0
+        //   256x32768 (524288)        7.6 / 9.0 / 9.6      6.8 / 7.7 / 8.4     13.2 / 13.5 / 14.2
+        //   64x16000  (64000)         3.1 / 2.4 / 3.5      3.2 / 3.0 / 3.7     10.0 / 10.3 / 10.7
+        // A small grid is done before a pipeline has filled; one big CTA a SM leaves SMs idle in its last
+        // round on images of few units, and its one copy queue is slow on short rows.
+        constexpr uint32_t kTinyBlocks = 20000, kTinyRow = 32, kBigBlocks = 600000, kBigRow = 256;
+        const uint32_t blocks = bw * bh;
+        if (access == SrcAccess::kVec16 && blocks >= kTinyBlocks && bw >= kTinyRow) {
+            if (tile.threads == 512 && tile.bpt == 2 && (blocks < kBigBlocks || bw < kBigRow)) tile = Tile{128, 1, 2};
             return launch_image_tma(codec, src, stride, dst, width, height, tile, stream, dst2);
-        tile.persistent = 0;  // word-aligned rows: the register-loading kernel with the same shape
+        }
+        // word-aligned rows take four times the load instructions and want many small CTAs at every size
+        // (4096^2 ETC1s, 2 blocks a thread: 16.4 us with 128 threads, 26.5 us with 512)
+        tile = Tile{128, access == SrcAccess::kWord4 && blocks >= kBigBlocks ? 2u : 1u, 0};
     }
     if (codec == kBC1) return launch_access<kBC1>(src, stride, dst, nullptr, bw, bh, tile, access, stream);
     if (codec == kETC1S) return launch_access<kETC1S>(src, stride, dst, nullptr, bw, bh, tile, access, stream);

@@ -1,17 +1,29 @@
 // encode_tma.cu -- the image encoder fed by bulk asynchronous copies.
 //
 // A resident grid of CTAs, each with one producer warp and C compute warps
-// (C = threads / 32).  Work is cut into tiles of 4 pixel rows x (32 * C * BPT)
-// blocks; CTA b takes tiles b, b + grid, ...  The producer's elected lane
-// copies each tile's four row segments (16 bytes per block, contiguous in the
-// source) into the next free stage of a shared-memory ring with
+// (C = threads / 32).  Work is cut into units of 32 * C * BPT consecutive
+// blocks of the image in row-major order; CTA b takes units b, b + grid, ...
+// The producer's elected lane copies each unit's pixel rows (16 bytes per
+// block, contiguous in the source; four pieces for every block row that the
+// unit touches) into the next free stage of a shared-memory ring with
 // cp.async.bulk, counted on that stage's "full" mbarrier; compute warps wait
 // for it, pull their blocks into registers with conflict-free 128-bit shared
-// loads (lane l of a warp reads 16 contiguous bytes, the warp 512), run the
+// loads (lane l of a warp reads 16 contiguous bytes, the warp 512: block k of
+// a unit lies at 16 * k of each of the stage's four planes, whatever rows it
+// came from), run the
 // same block codec as every other kernel, store 8 bytes per block with
 // streaming stores and release the stage on its "empty" mbarrier.  Global
 // loads never sit in the compute warps' registers, so the integer math of one
-// tile overlaps the HBM reads of the next stages.
+// unit overlaps the HBM reads of the next stages.
+//
+// Units run on across block rows, so every stage but the last is full at any
+// width.  Tiles that ended with their row left a stage half empty at 2048
+// pixels and added a nearly empty one to each row a little wider than a
+// stage: 4100x4096 BC1 16.7, ETC1s 20.1, both 24.6 us then, 11.1, 12.3 and
+// 14.7 us so (floor 11.3 us at 4.5 B/px of measured HBM; 4096^2 unchanged at
+// 11.0, 12.2 and 14.4 us).  The producer stays one lane: copies issued by
+// several lanes at once cost more (ETC1s 4096^2 12.5 us), and so did tiles
+// of several rows and part of the width (short row copies; 15.4 us).
 //
 // Launched with programmatic dependent launch (pdl.cuh): the prologue
 // (barriers, control-byte table) runs while the previous kernel in the stream
@@ -83,15 +95,14 @@ __host__ __device__ constexpr uint32_t l2_prefetch_tiles(const TmaLayout& l)
     return (uint32_t)GOOFY_L2_PREFETCH_TILES < l.stages ? (uint32_t)GOOFY_L2_PREFETCH_TILES : l.stages;
 }
 
-// Encodes the blocks of one stage held in shared memory (4 rows of
-// row_bytes, block b at 16 * b in each) and stores those below nb at
-// out + 8 * b (and out2, for both codecs).  Thread `lane` of compute warp
+// Encodes the blocks of one stage held in shared memory (four pixel rows of
+// row_bytes, block k of the unit at 16 * k in each) and stores those below nb
+// at out + 8 * k (and out2, for both codecs).  Thread `lane` of compute warp
 // `warp` takes blocks (warp * BPT + j) * 32 + lane.  Every thread loads and
-// encodes all its slots, also past nb (a narrower tile at the right edge):
-// such a slot holds whatever an earlier tile left in the stage, which
-// nothing writes while the stage is held, and its result is dropped.  Only
-// the stores are conditional, so the loads and the codec run without
-// branches.
+// encodes all its slots, also past nb (the image's last, shorter unit): such
+// a slot holds whatever an earlier unit left in the stage, which nothing
+// writes while the stage is held, and its result is dropped.  Only the
+// stores are conditional, so the loads and the codec run without branches.
 template <int CODEC, int BPT>
 __device__ __forceinline__ void encode_stage(const uint8_t* buf, uint32_t row_bytes, uint32_t warp, uint32_t lane,
                                              uint32_t nb, uint8_t* out, uint8_t* out2, const uint8_t* ctrl_lut)
@@ -125,11 +136,30 @@ __device__ __forceinline__ void encode_stage(const uint8_t* buf, uint32_t row_by
     }
 }
 
+// Calls f(k, nb, p) for every run of unit blocks [first, first + n) in one
+// block row of the image: unit blocks k .. k + nb - 1, whose first pixel row
+// starts at p.
+template <typename F>
+__device__ __forceinline__ void for_unit_rows(const uint8_t* src, size_t stride, uint32_t bw, uint32_t bw_magic,
+                                              uint32_t first, uint32_t n, F f)
+{
+    uint32_t bx;
+    const uint32_t by = div_magic(first, bw, bw_magic, bx);
+    const uint8_t* p = src + (size_t)by * 4u * stride + 16u * (size_t)bx;
+    uint32_t nb = min(bw - bx, n);
+    f(0u, nb, p);
+    for (uint32_t k = nb; k < n; k += nb) {
+        p += 4u * stride - 16u * (size_t)bx;
+        bx = 0u;
+        nb = min(bw, n - k);
+        f(k, nb, p);
+    }
+}
+
 template <int CODEC, int BPT, int COMPUTE>
 __global__ void __launch_bounds__(COMPUTE + 32, tma_min_ctas(BPT, COMPUTE))
     encode_image_tma(const uint8_t* __restrict__ src, size_t stride, uint8_t* __restrict__ dst,
-                     uint8_t* __restrict__ dst2, uint32_t bw, uint32_t tiles_per_row, uint32_t total_tiles,
-                     uint32_t tile_magic)
+                     uint8_t* __restrict__ dst2, uint32_t bw, uint32_t bw_magic, uint32_t total)
 {
     pdl_launch_dependents();
     extern __shared__ __align__(128) uint8_t smem[];
@@ -140,6 +170,8 @@ __global__ void __launch_bounds__(COMPUTE + 32, tma_min_ctas(BPT, COMPUTE))
     uint64_t* empty = full + L.stages;
     uint8_t* ctrl_lut = reinterpret_cast<uint8_t*>(empty + L.stages);
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+    constexpr uint32_t unit = L.tile_blocks;
+    const uint32_t step = gridDim.x * unit;  // units blockIdx.x, + gridDim.x, ...
 
     if (threadIdx.x == 0) {
         for (uint32_t s = 0; s < L.stages; ++s) {
@@ -153,19 +185,16 @@ __global__ void __launch_bounds__(COMPUTE + 32, tma_min_ctas(BPT, COMPUTE))
     __syncthreads();
     if (warp == compute_warps && lane == 0) {
         // While the previous kernel in the stream drains, ask L2 for the rows
-        // of this CTA's first tiles.  Only a hint: no data enters the CTA
+        // of this CTA's first units.  Only a hint: no data enters the CTA
         // before pdl_wait(), and L2 is coherent with the previous kernel's
         // writes, so the copies after the wait still read what it wrote.
-        uint32_t n = 0;
-        for (uint32_t t = blockIdx.x; t < total_tiles && n < l2_prefetch_tiles(L); t += gridDim.x, ++n) {
-            uint32_t tx;
-            const uint32_t by = div_magic(t, tiles_per_row, tile_magic, tx);
-            const uint32_t bx0 = tx * L.tile_blocks;
-            const uint32_t bytes = 16u * min(L.tile_blocks, bw - bx0);
-            const uint8_t* row = src + (size_t)by * 4u * stride + 16u * (size_t)bx0;
+        uint32_t c = 0;
+        for (uint32_t first = blockIdx.x * unit; first < total && c < l2_prefetch_tiles(L); first += step, ++c)
+            for_unit_rows(src, stride, bw, bw_magic, first, min(unit, total - first),
+                          [&](uint32_t, uint32_t nb, const uint8_t* row) {
 #pragma unroll
-            for (int r = 0; r < 4; ++r) bulk_prefetch_l2(row + r * stride, bytes);
-        }
+                              for (int r = 0; r < 4; ++r) bulk_prefetch_l2(row + r * stride, 16u * nb);
+                          });
     }
     pdl_wait();  // no global memory access before the previous kernel in the stream is done
 
@@ -177,20 +206,17 @@ __global__ void __launch_bounds__(COMPUTE + 32, tma_min_ctas(BPT, COMPUTE))
         // slower at 8192^2; with half, as fast there and 0.4 us faster at 4096^2.
         const uint64_t policy = CODEC == kBoth ? l2_evict_first_half_policy() : l2_evict_first_policy();
         uint32_t issued = 0, slot = 0, phase = 0;
-        for (uint32_t t = blockIdx.x; t < total_tiles; t += gridDim.x) {
+        for (uint32_t first = blockIdx.x * unit; first < total; first += step) {
             if (issued >= L.stages && !mbar_wait(&empty[slot], phase ^ 1u, &abort_flag, &g_pipeline_timeouts))
                 break;
-            uint32_t tx;
-            const uint32_t by = div_magic(t, tiles_per_row, tile_magic, tx);
-            const uint32_t bx0 = tx * L.tile_blocks;
-            const uint32_t nb = min(L.tile_blocks, bw - bx0);
-            const uint32_t bytes = 16u * nb;
-            mbar_arrive_expect_tx(&full[slot], 4u * bytes);
-            const uint8_t* row = src + (size_t)by * 4u * stride + 16u * (size_t)bx0;
+            const uint32_t n = min(unit, total - first);
+            mbar_arrive_expect_tx(&full[slot], 64u * n);
             uint8_t* buf = smem + slot * L.stage_bytes;
+            for_unit_rows(src, stride, bw, bw_magic, first, n, [&](uint32_t k, uint32_t nb, const uint8_t* row) {
 #pragma unroll
-            for (int r = 0; r < 4; ++r)
-                bulk_copy_g2s_hint(buf + r * L.row_bytes, row + r * stride, bytes, &full[slot], policy);
+                for (int r = 0; r < 4; ++r)
+                    bulk_copy_g2s_hint(buf + r * L.row_bytes + 16u * k, row + r * stride, 16u * nb, &full[slot], policy);
+            });
             ++issued;
             if (++slot == L.stages) {
                 slot = 0;
@@ -207,17 +233,14 @@ __global__ void __launch_bounds__(COMPUTE + 32, tma_min_ctas(BPT, COMPUTE))
     }
 
     uint32_t slot = 0, phase = 0;
-    for (uint32_t t = blockIdx.x; t < total_tiles; t += gridDim.x) {
+    for (uint32_t first = blockIdx.x * unit; first < total; first += step) {
         if (!mbar_wait(&full[slot], phase, &abort_flag, &g_pipeline_timeouts)) break;
-        uint32_t tx;
-        const uint32_t by = div_magic(t, tiles_per_row, tile_magic, tx);
-        const uint32_t bx0 = tx * L.tile_blocks;
-        const uint32_t nb = min(L.tile_blocks, bw - bx0);
+        const uint32_t nb = min(unit, total - first);
         const uint8_t* buf = smem + slot * L.stage_bytes;
-        const size_t o = ((size_t)by * bw + bx0) * 8u;
-        if (warp * (BPT * 32u) < nb)  // warps wholly past a narrower tile's last block skip it
-            encode_stage<CODEC, BPT>(buf, L.row_bytes, warp, lane, nb, dst + o,
-                                     CODEC == kBoth ? dst2 + o : nullptr, ctrl_lut);
+        const size_t o = (size_t)first * 8u;
+        if (warp * (BPT * 32u) < nb)  // warps wholly past the unit's last block skip it
+            encode_stage<CODEC, BPT>(buf, L.row_bytes, warp, lane, nb, dst + o, CODEC == kBoth ? dst2 + o : nullptr,
+                                     ctrl_lut);
         // Release the stage only now.  An arrival right after the shared loads
         // can overtake them: the loads wait in the load/store queue (behind
         // other kernels' global loads when SMs are shared) while the arrival
@@ -491,12 +514,12 @@ cudaError_t launch_tma_t(const uint8_t* src, size_t stride, uint8_t* dst, uint8_
         ctas = (sms > 0 ? sms : 1) * (per_sm > 0 ? per_sm : 1);
         resident[dev].store(ctas, std::memory_order_relaxed);
     }
-    const uint32_t tiles_per_row = (bw + L.tile_blocks - 1) / L.tile_blocks;
-    const uint64_t total = (uint64_t)tiles_per_row * bh;
-    if (total > 0x7fffffffull) return cudaErrorInvalidValue;
-    const uint32_t grid = (uint32_t)(total < (uint64_t)ctas ? total : (uint64_t)ctas);
+    const uint32_t total = bw * bh;
+    constexpr uint32_t unit = L.tile_blocks;
+    const uint32_t units = (total + unit - 1) / unit;
+    const uint32_t grid = units < (uint32_t)ctas ? units : (uint32_t)ctas;
     return launch_pdl(encode_image_tma<CODEC, BPT, COMPUTE>, dim3(grid), dim3(block), smem, stream, src, stride, dst,
-                      dst2, bw, tiles_per_row, (uint32_t)total, 0xffffffffu / tiles_per_row);
+                      dst2, bw, 0xffffffffu / bw, total);
 }
 
 template <int CODEC, int BPT>

@@ -13,6 +13,7 @@ struct Tile {
     uint32_t bpt;         // 4x4 blocks per thread and segment: 1, 2 or 4 (1 or 2 when persistent)
     uint32_t persistent;  // 0: one segment per warp; 1: resident grid looping over segments with prefetch;
                           // 2: resident grid fed by bulk copies into a shared-memory ring (+1 producer warp)
+                          //    for images large enough to fill it (launch_image), else shape 0
 };
 
 inline bool tile_valid(const Tile& t)

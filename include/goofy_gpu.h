@@ -137,9 +137,11 @@ typedef struct goofy_gpu_tile {
     uint32_t threads_per_cta;   /* 128, 256, 512 */
     uint32_t blocks_per_thread; /* 4x4 blocks a thread encodes per segment: 1, 2, 4 (1, 2 if persistent) */
     uint32_t persistent;        /* 0: one segment per warp; 1: resident grid, loop with prefetch;
-                                 * 2: resident grid, one producer warp streams tiles into a
+                                 * 2: resident grid, one producer warp streams runs of blocks into a
                                  *    shared-memory ring with bulk async copies (1, 2 blocks per
-                                 *    thread; 16-byte aligned sources, others run shape 0) */
+                                 *    thread).  Word-aligned sources and images of under 20,000 blocks
+                                 *    or 32 blocks a row run shape 0; 512 x 2 is the shape for large
+                                 *    images, smaller ones run it as 128 x 1 */
 } goofy_gpu_tile;
 
 /* Get / set the tile the image kernels launch with, per codec
