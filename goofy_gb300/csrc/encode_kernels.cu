@@ -243,13 +243,11 @@ cudaError_t launch_image(int codec, const uint8_t* src, size_t stride, uint8_t* 
         // round on images of few units, and its one copy queue is slow on short rows.
         constexpr uint32_t kTinyBlocks = 20000, kTinyRow = 32, kBigBlocks = 600000, kBigRow = 256;
         const uint32_t blocks = bw * bh;
-        if (access == SrcAccess::kVec16 && blocks >= kTinyBlocks && bw >= kTinyRow) {
+        if (blocks >= kTinyBlocks && bw >= kTinyRow) {
             if (tile.threads == 512 && tile.bpt == 2 && (blocks < kBigBlocks || bw < kBigRow)) tile = Tile{128, 1, 2};
-            return launch_image_tma(codec, src, stride, dst, width, height, tile, stream, dst2);
+            return launch_image_tma(codec, src, stride, dst, width, height, tile, access, stream, dst2);
         }
-        // word-aligned rows take four times the load instructions and want many small CTAs at every size
-        // (4096^2 ETC1s, 2 blocks a thread: 16.4 us with 128 threads, 26.5 us with 512)
-        tile = Tile{128, access == SrcAccess::kWord4 && blocks >= kBigBlocks ? 2u : 1u, 0};
+        tile = Tile{128, 1, 0};
     }
     if (codec == kBC1) return launch_access<kBC1>(src, stride, dst, nullptr, bw, bh, tile, access, stream);
     if (codec == kETC1S) return launch_access<kETC1S>(src, stride, dst, nullptr, bw, bh, tile, access, stream);

@@ -29,8 +29,13 @@
 // (barriers, control-byte table) runs while the previous kernel in the stream
 // drains, and no copy is issued before that kernel has completed.
 //
-// Needs 16-byte aligned source rows (base and stride); other images take the
-// register-loading kernels.  Every wait is bounded (async_copy.cuh): a stuck
+// Word-aligned rows (a part of an atlas at an odd pixel offset, a padded
+// stride) take the same kernel: whole 16-byte granules are copied and the
+// shift is taken out when the words leave shared memory.  The
+// register-loading kernel reads such a block with sixteen 4-byte loads that
+// skip L1, so every 32-byte sector crosses L2 up to four times: 1996x1532
+// ETC1s 7.3-11.0 us there, 5.2 us here; 4096^2 (over 400 MB of inputs) BC1 15.8,
+// ETC1s 17.0 there with the best CTA size, 13.1 and 14.1 here.  Every wait is bounded (async_copy.cuh): a stuck
 // barrier ends the kernel with a counted time-out instead of a hang, and the
 // producer then waits (bounded) for the copies it issued before its CTA exits.
 #include <cuda_runtime.h>
@@ -64,17 +69,24 @@ struct TmaLayout {
     uint32_t tile_blocks, row_bytes, stage_bytes, stages;
 };
 
-__host__ __device__ constexpr TmaLayout tma_layout(uint32_t compute_threads, uint32_t bpt)
+// Word-aligned rows: a run of nb blocks is copied as the 16-byte granules that
+// hold it, up to nb + 1 of them, so every plane has room for one more granule
+// per block row that a unit touches (and the one read past the last block).
+// kWordSlack of them serve units of up to 5 block rows' width.
+constexpr uint32_t kWordSlack = 8;
+__host__ __device__ constexpr bool word_rows_fit(uint32_t tile_blocks, uint32_t bw) { return tile_blocks <= 5u * bw; }
+
+__host__ __device__ constexpr TmaLayout tma_layout(uint32_t compute_threads, uint32_t bpt, bool word = false)
 {
     TmaLayout l{};
     l.tile_blocks = compute_threads * bpt;
-    l.row_bytes = 16u * l.tile_blocks;
+    l.row_bytes = 16u * (l.tile_blocks + (word ? kWordSlack : 0u));
     l.stage_bytes = 4u * l.row_bytes;
     // ring budget scaled with the CTA (112 KB at 512 compute threads), so the
     // CTAs the registers allow per SM also fit in shared memory; at least 3
     // stages for a CTA alone on its SM (a stage is released only once it has
     // been encoded, so 2 would leave that SM a single stage of lookahead)
-    const uint32_t s = (114688u / 512u * compute_threads) / l.stage_bytes;
+    const uint32_t s = (114688u / 512u * compute_threads) / (64u * l.tile_blocks);
     const uint32_t lo = tma_min_ctas(bpt, compute_threads) == 1 ? 3u : 2u;
     l.stages = s < lo ? lo : s > 6u ? 6u : s;
     return l;
@@ -103,21 +115,39 @@ __host__ __device__ constexpr uint32_t l2_prefetch_tiles(const TmaLayout& l)
 // a slot holds whatever an earlier unit left in the stage, which nothing
 // writes while the stage is held, and its result is dropped.  Only the
 // stores are conditional, so the loads and the codec run without branches.
-template <int CODEC, int BPT>
+// WORD: block k's pixel row y starts shift[y] bytes into granule
+// k + (its block row - the unit's first) of plane y and is read word by word
+// (four lanes a bank, 64 wavefronts a warp and block instead of 16, which the
+// load/store unit has room for; picking the words out of two 16-byte loads
+// would take 36 selects a block on the busy ALU pipe).
+template <int CODEC, int BPT, bool WORD>
 __device__ __forceinline__ void encode_stage(const uint8_t* buf, uint32_t row_bytes, uint32_t warp, uint32_t lane,
-                                             uint32_t nb, uint8_t* out, uint8_t* out2, const uint8_t* ctrl_lut)
+                                             uint32_t nb, uint8_t* out, uint8_t* out2, const uint8_t* ctrl_lut,
+                                             uint32_t bx0, uint32_t bw, uint32_t bw_magic,
+                                             const uint32_t (&shift)[4])
 {
     uint32_t w[BPT][16];
 #pragma unroll
     for (int j = 0; j < BPT; ++j) {
         const uint32_t b = (warp * BPT + j) * 32u + lane;
+        if constexpr (WORD) {
+            uint32_t x;
+            const uint32_t s = div_magic(min(bx0 + b, bx0 + nb - 1u), bw, bw_magic, x);
+            const uint8_t* p = buf + 16u * (min(b, nb - 1u) + s);
 #pragma unroll
-        for (int r = 0; r < 4; ++r) {
-            const uint4 v = *reinterpret_cast<const uint4*>(buf + r * row_bytes + 16u * b);
-            w[j][4 * r + 0] = v.x;
-            w[j][4 * r + 1] = v.y;
-            w[j][4 * r + 2] = v.z;
-            w[j][4 * r + 3] = v.w;
+            for (int r = 0; r < 4; ++r)
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    w[j][4 * r + i] = *reinterpret_cast<const uint32_t*>(p + r * row_bytes + shift[r] + 4 * i);
+        } else {
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                const uint4 v = *reinterpret_cast<const uint4*>(buf + r * row_bytes + 16u * b);
+                w[j][4 * r + 0] = v.x;
+                w[j][4 * r + 1] = v.y;
+                w[j][4 * r + 2] = v.z;
+                w[j][4 * r + 3] = v.w;
+            }
         }
     }
 #pragma unroll
@@ -156,7 +186,12 @@ __device__ __forceinline__ void for_unit_rows(const uint8_t* src, size_t stride,
     }
 }
 
-template <int CODEC, int BPT, int COMPUTE>
+// WORD: the rows are only 4-byte aligned.  4 * stride is then a multiple of
+// 16, so pixel row y of every block row starts shift[y] = (src + y * stride)
+// % 16 bytes past a 16-byte boundary; the copies take whole granules from that
+// boundary on (the first and last may hold bytes of other pixels, never of
+// another allocation's page) and the compute warps read at the shift.
+template <int CODEC, int BPT, int COMPUTE, bool WORD>
 __global__ void __launch_bounds__(COMPUTE + 32, tma_min_ctas(BPT, COMPUTE))
     encode_image_tma(const uint8_t* __restrict__ src, size_t stride, uint8_t* __restrict__ dst,
                      uint8_t* __restrict__ dst2, uint32_t bw, uint32_t bw_magic, uint32_t total)
@@ -165,13 +200,18 @@ __global__ void __launch_bounds__(COMPUTE + 32, tma_min_ctas(BPT, COMPUTE))
     extern __shared__ __align__(128) uint8_t smem[];
     __shared__ uint32_t abort_flag;
     constexpr uint32_t compute_warps = COMPUTE / 32;
-    constexpr TmaLayout L = tma_layout(COMPUTE, BPT);
+    constexpr TmaLayout L = tma_layout(COMPUTE, BPT, WORD);
     uint64_t* full = reinterpret_cast<uint64_t*>(smem + L.stages * L.stage_bytes);
     uint64_t* empty = full + L.stages;
     uint8_t* ctrl_lut = reinterpret_cast<uint8_t*>(empty + L.stages);
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
     constexpr uint32_t unit = L.tile_blocks;
     const uint32_t step = gridDim.x * unit;  // units blockIdx.x, + gridDim.x, ...
+    uint32_t shift[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) shift[r] = WORD ? (uint32_t)(reinterpret_cast<uintptr_t>(src) + r * stride) & 15u : 0u;
+    // bytes of pixel row r's piece of nb blocks
+    auto piece = [&](uint32_t nb, int r) { return WORD ? (16u * nb + shift[r] + 15u) & ~15u : 16u * nb; };
 
     if (threadIdx.x == 0) {
         for (uint32_t s = 0; s < L.stages; ++s) {
@@ -193,7 +233,7 @@ __global__ void __launch_bounds__(COMPUTE + 32, tma_min_ctas(BPT, COMPUTE))
             for_unit_rows(src, stride, bw, bw_magic, first, min(unit, total - first),
                           [&](uint32_t, uint32_t nb, const uint8_t* row) {
 #pragma unroll
-                              for (int r = 0; r < 4; ++r) bulk_prefetch_l2(row + r * stride, 16u * nb);
+                              for (int r = 0; r < 4; ++r) bulk_prefetch_l2(row + r * stride - shift[r], piece(nb, r));
                           });
     }
     pdl_wait();  // no global memory access before the previous kernel in the stream is done
@@ -210,12 +250,22 @@ __global__ void __launch_bounds__(COMPUTE + 32, tma_min_ctas(BPT, COMPUTE))
             if (issued >= L.stages && !mbar_wait(&empty[slot], phase ^ 1u, &abort_flag, &g_pipeline_timeouts))
                 break;
             const uint32_t n = min(unit, total - first);
-            mbar_arrive_expect_tx(&full[slot], 64u * n);
+            uint32_t bytes = 64u * n, s = 0;
+            if constexpr (WORD) {
+                bytes = 0;
+                for_unit_rows(src, stride, bw, bw_magic, first, n, [&](uint32_t, uint32_t nb, const uint8_t*) {
+#pragma unroll
+                    for (int r = 0; r < 4; ++r) bytes += piece(nb, r);
+                });
+            }
+            mbar_arrive_expect_tx(&full[slot], bytes);
             uint8_t* buf = smem + slot * L.stage_bytes;
             for_unit_rows(src, stride, bw, bw_magic, first, n, [&](uint32_t k, uint32_t nb, const uint8_t* row) {
 #pragma unroll
                 for (int r = 0; r < 4; ++r)
-                    bulk_copy_g2s_hint(buf + r * L.row_bytes + 16u * k, row + r * stride, 16u * nb, &full[slot], policy);
+                    bulk_copy_g2s_hint(buf + r * L.row_bytes + 16u * (k + s), row + r * stride - shift[r],
+                                       piece(nb, r), &full[slot], policy);
+                if constexpr (WORD) ++s;
             });
             ++issued;
             if (++slot == L.stages) {
@@ -238,9 +288,11 @@ __global__ void __launch_bounds__(COMPUTE + 32, tma_min_ctas(BPT, COMPUTE))
         const uint32_t nb = min(unit, total - first);
         const uint8_t* buf = smem + slot * L.stage_bytes;
         const size_t o = (size_t)first * 8u;
+        uint32_t bx0 = 0;
+        if constexpr (WORD) div_magic(first, bw, bw_magic, bx0);
         if (warp * (BPT * 32u) < nb)  // warps wholly past the unit's last block skip it
-            encode_stage<CODEC, BPT>(buf, L.row_bytes, warp, lane, nb, dst + o, CODEC == kBoth ? dst2 + o : nullptr,
-                                     ctrl_lut);
+            encode_stage<CODEC, BPT, WORD>(buf, L.row_bytes, warp, lane, nb, dst + o,
+                                           CODEC == kBoth ? dst2 + o : nullptr, ctrl_lut, bx0, bw, bw_magic, shift);
         // Release the stage only now.  An arrival right after the shared loads
         // can overtake them: the loads wait in the load/store queue (behind
         // other kernels' global loads when SMs are shared) while the arrival
@@ -485,11 +537,11 @@ __global__ void __launch_bounds__(COMPUTE + 32, tma_min_ctas(BPT, COMPUTE))
 
 namespace {
 
-template <int CODEC, int BPT, int COMPUTE>
+template <int CODEC, int BPT, int COMPUTE, bool WORD>
 cudaError_t launch_tma_t(const uint8_t* src, size_t stride, uint8_t* dst, uint8_t* dst2, uint32_t bw, uint32_t bh,
                          cudaStream_t stream)
 {
-    constexpr TmaLayout L = tma_layout(COMPUTE, BPT);
+    constexpr TmaLayout L = tma_layout(COMPUTE, BPT, WORD);
     const size_t smem = tma_smem_bytes(L);
     constexpr uint32_t block = COMPUTE + 32u;
     // per device: dynamic shared memory opt-in and resident CTAs per SM
@@ -500,15 +552,15 @@ cudaError_t launch_tma_t(const uint8_t* src, size_t stride, uint8_t* dst, uint8_
     if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
     int ctas = resident[dev].load(std::memory_order_relaxed);
     if (ctas == 0) {
-        e = cudaFuncSetAttribute(encode_image_tma<CODEC, BPT, COMPUTE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        e = cudaFuncSetAttribute(encode_image_tma<CODEC, BPT, COMPUTE, WORD>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)smem);
         if (e != cudaSuccess) return e;
-        e = cudaFuncSetAttribute(encode_image_tma<CODEC, BPT, COMPUTE>,
+        e = cudaFuncSetAttribute(encode_image_tma<CODEC, BPT, COMPUTE, WORD>,
                                  cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
         if (e != cudaSuccess) return e;
         int sms = 0, per_sm = 0;
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, encode_image_tma<CODEC, BPT, COMPUTE>, (int)block,
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, encode_image_tma<CODEC, BPT, COMPUTE, WORD>, (int)block,
                                                           smem);
         if (e != cudaSuccess) return e;
         ctas = (sms > 0 ? sms : 1) * (per_sm > 0 ? per_sm : 1);
@@ -518,7 +570,7 @@ cudaError_t launch_tma_t(const uint8_t* src, size_t stride, uint8_t* dst, uint8_
     constexpr uint32_t unit = L.tile_blocks;
     const uint32_t units = (total + unit - 1) / unit;
     const uint32_t grid = units < (uint32_t)ctas ? units : (uint32_t)ctas;
-    return launch_pdl(encode_image_tma<CODEC, BPT, COMPUTE>, dim3(grid), dim3(block), smem, stream, src, stride, dst,
+    return launch_pdl(encode_image_tma<CODEC, BPT, COMPUTE, WORD>, dim3(grid), dim3(block), smem, stream, src, stride, dst,
                       dst2, bw, 0xffffffffu / bw, total);
 }
 
@@ -527,28 +579,47 @@ cudaError_t launch_tma_bpt(const uint8_t* src, size_t stride, uint8_t* dst, uint
                            uint32_t threads, cudaStream_t stream)
 {
     switch (threads) {
-    case 128: return launch_tma_t<CODEC, BPT, 128>(src, stride, dst, dst2, bw, bh, stream);
-    case 256: return launch_tma_t<CODEC, BPT, 256>(src, stride, dst, dst2, bw, bh, stream);
-    case 512: return launch_tma_t<CODEC, BPT, 512>(src, stride, dst, dst2, bw, bh, stream);
+    case 128: return launch_tma_t<CODEC, BPT, 128, false>(src, stride, dst, dst2, bw, bh, stream);
+    case 256: return launch_tma_t<CODEC, BPT, 256, false>(src, stride, dst, dst2, bw, bh, stream);
+    case 512: return launch_tma_t<CODEC, BPT, 512, false>(src, stride, dst, dst2, bw, bh, stream);
     default: return cudaErrorInvalidValue;
     }
+}
+
+// Word-aligned rows come in two shapes, 512 x 2 and 128 x 1.
+template <int CODEC>
+cudaError_t launch_tma_word(const uint8_t* src, size_t stride, uint8_t* dst, uint8_t* dst2, uint32_t bw, uint32_t bh,
+                            bool big, cudaStream_t stream)
+{
+    return big ? launch_tma_t<CODEC, 2, 512, true>(src, stride, dst, dst2, bw, bh, stream)
+               : launch_tma_t<CODEC, 1, 128, true>(src, stride, dst, dst2, bw, bh, stream);
 }
 
 }  // namespace
 
 cudaError_t launch_image_tma(int codec, const uint8_t* src, size_t stride, uint8_t* dst, uint32_t width,
-                             uint32_t height, Tile tile, cudaStream_t stream, uint8_t* dst2)
+                             uint32_t height, Tile tile, SrcAccess access, cudaStream_t stream, uint8_t* dst2)
 {
     const uint32_t bw = width / 4, bh = height / 4;
     if (bw == 0 || bh == 0) return cudaSuccess;
-    if (reinterpret_cast<uintptr_t>(src) % 16 || stride % 16) return cudaErrorInvalidValue;
+    const uint32_t align = access == SrcAccess::kVec16 ? 16 : 4;
+    if (reinterpret_cast<uintptr_t>(src) % align || stride % align) return cudaErrorInvalidValue;
+    if (codec == kBoth && !dst2) return cudaErrorInvalidValue;
+    if (access == SrcAccess::kWord4) {
+        const bool big = tile.threads == 512 && tile.bpt == 2;
+        if (!word_rows_fit(big ? 1024 : 128, bw)) return cudaErrorInvalidValue;
+        if (codec == kBC1) return launch_tma_word<kBC1>(src, stride, dst, nullptr, bw, bh, big, stream);
+        if (codec == kETC1S) return launch_tma_word<kETC1S>(src, stride, dst, nullptr, bw, bh, big, stream);
+        if (codec == kBoth) return launch_tma_word<kBoth>(src, stride, dst, dst2, bw, bh, big, stream);
+        return cudaErrorInvalidValue;
+    }
     if (codec == kBC1) {
         if (tile.bpt == 1) return launch_tma_bpt<kBC1, 1>(src, stride, dst, nullptr, bw, bh, tile.threads, stream);
         if (tile.bpt == 2) return launch_tma_bpt<kBC1, 2>(src, stride, dst, nullptr, bw, bh, tile.threads, stream);
     } else if (codec == kETC1S) {
         if (tile.bpt == 1) return launch_tma_bpt<kETC1S, 1>(src, stride, dst, nullptr, bw, bh, tile.threads, stream);
         if (tile.bpt == 2) return launch_tma_bpt<kETC1S, 2>(src, stride, dst, nullptr, bw, bh, tile.threads, stream);
-    } else if (codec == kBoth && dst2) {
+    } else if (codec == kBoth) {
         if (tile.bpt == 1) return launch_tma_bpt<kBoth, 1>(src, stride, dst, dst2, bw, bh, tile.threads, stream);
         if (tile.bpt == 2) return launch_tma_bpt<kBoth, 2>(src, stride, dst, dst2, bw, bh, tile.threads, stream);
     }

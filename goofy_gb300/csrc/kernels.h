@@ -37,10 +37,12 @@ enum class SrcAccess : int {
 cudaError_t launch_image(int codec, const uint8_t* src, size_t stride, uint8_t* dst, uint32_t width,
                          uint32_t height, Tile tile, SrcAccess access, cudaStream_t stream, uint8_t* dst2 = nullptr);
 
-// The bulk-copy pipeline kernel (tile.persistent == 2); needs a 16-byte
-// aligned source base and stride.
+// The bulk-copy pipeline kernel (tile.persistent == 2).  Word-aligned sources
+// (kWord4) run it with 512 x 2 tiles (rows of 205 blocks or more) or, for any
+// other tile, 128 x 1 (rows of 26 or more).  Device memory only.
 cudaError_t launch_image_tma(int codec, const uint8_t* src, size_t stride, uint8_t* dst, uint32_t width,
-                             uint32_t height, Tile tile, cudaStream_t stream, uint8_t* dst2 = nullptr);
+                             uint32_t height, Tile tile, SrcAccess access, cudaStream_t stream,
+                             uint8_t* dst2 = nullptr);
 
 // Pipeline waits that gave up on the current device since the last reset.
 cudaError_t pipeline_timeouts(unsigned int* count, bool reset);

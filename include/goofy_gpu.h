@@ -57,7 +57,8 @@ const char* goofy_gpu_last_error(void);
 
 /* Device-pointer variant of goofy::compressDXT1 (goofy_tc.h:1497-1526).
  * src: device RGBA8, `stride` bytes per row (4-byte aligned; 16-byte aligned
- * src and stride take the vector-load path).  dst: device, 8-byte aligned,
+ * src and stride are fastest; reads whole 16-byte granules of device memory,
+ * so up to 12 bytes before and after the rows, and uses none of them).  dst: device, 8-byte aligned,
  * (width/4)*(height/4)*8 bytes.  width % 4 == 0 (not % 16: blocks are
  * independent), height % 4 == 0.  Enqueues one kernel on `stream`; no sync.
  * The kernel is launched with programmatic stream serialization: after one of
@@ -139,9 +140,10 @@ typedef struct goofy_gpu_tile {
     uint32_t persistent;        /* 0: one segment per warp; 1: resident grid, loop with prefetch;
                                  * 2: resident grid, one producer warp streams runs of blocks into a
                                  *    shared-memory ring with bulk async copies (1, 2 blocks per
-                                 *    thread).  Word-aligned sources and images of under 20,000 blocks
-                                 *    or 32 blocks a row run shape 0; 512 x 2 is the shape for large
-                                 *    images, smaller ones run it as 128 x 1 */
+                                 *    thread).  Images of under 20,000 blocks or 32 blocks a row run
+                                 *    shape 0; 512 x 2 is the shape for large images, smaller ones
+                                 *    run it as 128 x 1, and so do word-aligned sources of other
+                                 *    mode 2 shapes */
 } goofy_gpu_tile;
 
 /* Get / set the tile the image kernels launch with, per codec

@@ -64,3 +64,34 @@ def test_bulk_copy_tiles_on_ragged_rows(cuda, threads, bpt):
         _check(cuda, img, w, h, stride, want)
     finally:
         g.reset_tiles()
+
+
+@pytest.mark.parametrize("w,h", [(564, 564), (568, 564), (124, 4000), (128, 4000), (1028, 2412), (3204, 3004),
+                                 (1020, 10000), (16384, 148)])
+@pytest.mark.parametrize("offset,pad", [(4, 0), (8, 4), (12, 8), (0, 12), (4, 20)])
+def test_word_aligned_rows(cuda, w, h, offset, pad):
+    """Rows that start 4, 8 or 12 bytes past a 16-byte boundary, the same for
+    every row (pad % 16 == 0) or changing from row to row."""
+    rng = np.random.default_rng(w + h)
+    stride = 4 * w + pad
+    img = np.zeros((h, stride), np.uint8)
+    img[:, :4 * w] = workloads.scene(w, h, seed=w + offset)
+    img[:, 4 * w:] = rng.integers(0, 256, (h, pad), np.uint8)
+    want = [oracle.encode(c, img, w, h, stride) for c in (g.CODEC_BC1, g.CODEC_ETC1S)]
+    raw = cuda.empty(h * stride + 64, dtype=cuda.uint8, device="cuda").random_(0, 256)
+    src = raw[offset:offset + h * stride]
+    src.copy_(cuda.from_numpy(img.reshape(-1)).cuda())
+    stream = cuda.cuda.current_stream().cuda_stream
+    n = g.out_size(w, h)
+    for codec in (g.CODEC_BC1, g.CODEC_ETC1S):
+        dst = cuda.full((n + 64,), 0xA5, dtype=cuda.uint8, device="cuda")
+        assert g.compress_device(codec, dst, src, w, h, stride, stream) == g.OK, g.last_error()
+        got = dst.cpu().numpy()
+        np.testing.assert_array_equal(got[:n], want[codec])
+        assert (got[n:] == 0xA5).all()
+    both = cuda.zeros(2 * n, dtype=cuda.uint8, device="cuda")
+    assert g.compress_both_device(both.data_ptr(), both.data_ptr() + n, src, w, h, stride, stream) == g.OK
+    got = both.cpu().numpy()
+    np.testing.assert_array_equal(got[:n], want[0])
+    np.testing.assert_array_equal(got[n:], want[1])
+    assert g.pipeline_timeouts() == 0
