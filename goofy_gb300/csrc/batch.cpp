@@ -19,6 +19,7 @@
 
 #include <algorithm>
 #include <cstring>
+#include <memory>
 #include <mutex>
 #include <new>
 #include <vector>
@@ -60,43 +61,93 @@ struct goofy_gpu_batch {
     cudaStream_t stream = nullptr;
     Slot slot[2];
     int next = 0;
-    std::vector<uint32_t> units_scratch;
+    std::unique_ptr<goofy_gpu::ParamImage[]> table;  // of a call whose launches carry their descriptors
 };
+
+// Such a call is split into at most this many launches; larger ones upload
+// (a third launch costs what the upload does, batch_kernels.cu).
+constexpr uint32_t kParamLaunches = 2;
+
+namespace {
+
+constexpr uint64_t kResidentWarps = 152 * 64;
+
+// Checks one image and fills its descriptor (all zero for an empty image).
+int check_image(const goofy_gpu_image& im, BatchImage* out)
+{
+    if (im.codec != GOOFY_CODEC_BC1 && im.codec != GOOFY_CODEC_ETC1S)
+        return goofy_gpu::fail(GOOFY_ERR_INVALID, "batch: bad codec");
+    if (im.width % 4) return goofy_gpu::fail(GOOFY_ERR_WIDTH, "batch: width % 4 != 0");
+    if (im.height % 4) return goofy_gpu::fail(GOOFY_ERR_HEIGHT, "batch: height % 4 != 0");
+    const uint64_t bw = im.width / 4, bh = im.height / 4;
+    if (bw * bh > 0x7fffffffull) return goofy_gpu::fail(GOOFY_ERR_TOO_LARGE, "batch: image too large");
+    BatchImage& d = *out;
+    std::memset(&d, 0, sizeof d);
+    if (bw == 0 || bh == 0) return GOOFY_OK;
+    if (!im.src || !im.dst) return goofy_gpu::fail(GOOFY_ERR_INVALID, "batch: null pointer");
+    if ((uint64_t)im.stride < 4ull * im.width) return goofy_gpu::fail(GOOFY_ERR_INVALID, "batch: stride");
+    const uintptr_t s = reinterpret_cast<uintptr_t>(im.src);
+    if (reinterpret_cast<uintptr_t>(im.dst) % 8 || s % 4 || im.stride % 4)
+        return goofy_gpu::fail(GOOFY_ERR_ALIGNMENT, "batch: alignment");
+    d.src = static_cast<const uint8_t*>(im.src);
+    d.dst = static_cast<uint8_t*>(im.dst);
+    d.stride = im.stride;
+    d.bw = (uint32_t)bw;
+    d.bh = (uint32_t)bh;
+    d.bw_magic = 0xffffffffu / (uint32_t)bw;
+    d.codec = (uint32_t)im.codec;
+    d.vec16 = (s % 16 == 0 && im.stride % 16 == 0) ? 1u : 0u;
+    return GOOFY_OK;
+}
+
+int add_units(uint64_t blocks, uint32_t unit_blocks, uint64_t* units)
+{
+    *units += (blocks + unit_blocks - 1) / unit_blocks;
+    return *units > 0x7fffffffull ? goofy_gpu::fail(GOOFY_ERR_TOO_LARGE, "batch: too many work units") : GOOFY_OK;
+}
+
+}  // namespace
 
 int goofy_gpu::validate_and_fill(const goofy_gpu_image* images, uint32_t count, uint32_t unit_blocks,
                                  BatchImage* desc, uint32_t* first, uint32_t* total_units)
 {
     uint64_t units = 0;
     for (uint32_t i = 0; i < count; ++i) {
-        const goofy_gpu_image& im = images[i];
-        if (im.codec != GOOFY_CODEC_BC1 && im.codec != GOOFY_CODEC_ETC1S)
-            return goofy_gpu::fail(GOOFY_ERR_INVALID, "batch: bad codec");
-        if (im.width % 4) return goofy_gpu::fail(GOOFY_ERR_WIDTH, "batch: width % 4 != 0");
-        if (im.height % 4) return goofy_gpu::fail(GOOFY_ERR_HEIGHT, "batch: height % 4 != 0");
-        const uint64_t bw = im.width / 4, bh = im.height / 4;
-        if (bw * bh > 0x7fffffffull) return goofy_gpu::fail(GOOFY_ERR_TOO_LARGE, "batch: image too large");
-        BatchImage& d = desc[i];
-        std::memset(&d, 0, sizeof d);
-        d.first_unit = (uint32_t)units;
-        first[i] = (uint32_t)units;
-        if (bw == 0 || bh == 0) continue;  // empty image: no units
-        if (!im.src || !im.dst) return goofy_gpu::fail(GOOFY_ERR_INVALID, "batch: null pointer");
-        if ((uint64_t)im.stride < 4ull * im.width) return goofy_gpu::fail(GOOFY_ERR_INVALID, "batch: stride");
-        const uintptr_t s = reinterpret_cast<uintptr_t>(im.src);
-        if (reinterpret_cast<uintptr_t>(im.dst) % 8 || s % 4 || im.stride % 4)
-            return goofy_gpu::fail(GOOFY_ERR_ALIGNMENT, "batch: alignment");
-        d.src = static_cast<const uint8_t*>(im.src);
-        d.dst = static_cast<uint8_t*>(im.dst);
-        d.stride = im.stride;
-        d.bw = (uint32_t)bw;
-        d.bh = (uint32_t)bh;
-        d.bw_magic = 0xffffffffu / (uint32_t)bw;
-        d.codec = (uint32_t)im.codec;
-        d.vec16 = (s % 16 == 0 && im.stride % 16 == 0) ? 1u : 0u;
-        units += (bw * bh + unit_blocks - 1) / unit_blocks;
-        if (units > 0x7fffffffull) return goofy_gpu::fail(GOOFY_ERR_TOO_LARGE, "batch: too many work units");
+        int rc = check_image(images[i], &desc[i]);
+        if (rc != GOOFY_OK) return rc;
+        desc[i].first_unit = first[i] = (uint32_t)units;
+        if ((rc = add_units((uint64_t)desc[i].bw * desc[i].bh, unit_blocks, &units)) != GOOFY_OK) return rc;
     }
     *total_units = (uint32_t)units;
+    return GOOFY_OK;
+}
+
+int goofy_gpu::validate_and_fill(const goofy_gpu_image* images, uint32_t count, const BatchTile& tile, ParamLaunch* l)
+{
+    // Guided unit sizes: an image gets the largest units that still leave one for each of the GPU's warps
+    // among the blocks from it on, so the launch ends in small ones; between one pass of a warp's lanes and
+    // four of the tile's units.  A launch that fills the GPU many times over does not go below 128 blocks,
+    // where finding a unit's image begins to cost more than an even end saves.
+    const uint64_t pass = 32u * tile.bpt;
+    uint64_t left = 0, units = 0;
+    for (uint32_t i = 0; i < count; ++i) left += (uint64_t)(images[i].width / 4) * (images[i].height / 4);
+    uint32_t most = 0, least = 0;
+    while (most < 15 && pass << (most + 1) <= 4ull * tile.unit_blocks) ++most;
+    while (least < most && pass << (least + 1) <= 128 && (pass << (least + 1)) * kResidentWarps <= left) ++least;
+    for (uint32_t i = 0; i < count; ++i) {
+        BatchImage d;
+        int rc = check_image(images[i], &d);
+        if (rc != GOOFY_OK) return rc;
+        uint32_t c = most;
+        while (c > least && (pass << c) * kResidentWarps > left) --c;
+        const uint64_t blocks = (uint64_t)d.bw * d.bh;
+        l->images[i] = ParamImage{d.src, d.dst, d.stride, d.bw | d.codec << 28 | d.vec16 << 29 | (c & 3u) << 30,
+                                  d.bh | (c >> 2) << 30, (uint32_t)units};
+        if ((rc = add_units(blocks, (uint32_t)(pass << c), &units)) != GOOFY_OK) return rc;
+        left -= blocks;
+    }
+    l->count = count;
+    l->units = (uint32_t)units;
     return GOOFY_OK;
 }
 
@@ -126,6 +177,25 @@ cudaError_t enqueue(const Slot& s, uint32_t count, uint32_t units, const BatchTi
     return e;
 }
 
+// Launches that carry their descriptors (every image is checked before the first).
+int encode_params(goofy_gpu_batch* b, const goofy_gpu_image* images, uint32_t count, cudaStream_t caller,
+                  const BatchTile& tile)
+{
+    const uint32_t launches = (count + goofy_gpu::kParamImages - 1) / goofy_gpu::kParamImages;
+    goofy_gpu::ParamLaunch l[kParamLaunches];
+    for (uint32_t k = 0; k < launches; ++k) {
+        const uint32_t at = k * goofy_gpu::kParamImages;
+        l[k].images = &b->table[at];
+        const int rc = validate_and_fill(images + at, std::min(count - at, goofy_gpu::kParamImages), tile, &l[k]);
+        if (rc != GOOFY_OK) return rc;
+    }
+    for (uint32_t k = 0; k < launches; ++k) {
+        const cudaError_t e = goofy_gpu::launch_batch_params(l[k], tile, caller);
+        if (e != cudaSuccess) return cuda_fail(e, "batch launch");
+    }
+    return GOOFY_OK;
+}
+
 int encode_locked(goofy_gpu_batch* b, const goofy_gpu_image* images, uint32_t count, cudaStream_t caller,
                   const BatchTile& tile)
 {
@@ -146,6 +216,8 @@ int encode_locked(goofy_gpu_batch* b, const goofy_gpu_image* images, uint32_t co
         if (e != cudaSuccess) return cuda_fail(e, "batch launch");
         return GOOFY_OK;
     }
+    if (!tile.pipeline && count <= kParamLaunches * goofy_gpu::kParamImages)
+        return encode_params(b, images, count, caller, tile);
     Slot& s = b->slot[b->next];
     b->next ^= 1;
     if (s.in_flight) {
@@ -219,6 +291,11 @@ GOOFY_EXPORT int goofy_gpu_batch_create(goofy_gpu_batch** out, uint32_t max_imag
     if (!b) return GOOFY_ERR_NOMEM;
     b->device = device;
     b->max_images = max_images;
+    b->table.reset(new (std::nothrow) goofy_gpu::ParamImage[kParamLaunches * goofy_gpu::kParamImages]);
+    if (!b->table) {
+        delete b;
+        return GOOFY_ERR_NOMEM;
+    }
     auto cleanup = [&](int rc) {
         for (auto& s : b->slot) free_slot(s);
         if (b->stream) cudaStreamDestroy(b->stream);

@@ -61,6 +61,37 @@ struct InlineBatch {
 cudaError_t launch_batch_tma_inline(const InlineBatch& batch, uint32_t n_images, uint32_t total_units,
                                     const BatchTile& tile, uint32_t ctas, cudaStream_t stream);
 
+// A batch image as the parameter of the work-unit kernel: the same in 32
+// bytes, so that one launch carries 1022 of them (32,704 of the 32,764 bytes
+// that a kernel may take).  Flags sit in bits that sizes cannot reach: a row
+// has fewer than 2^28 blocks (its stride is 32 bits), an image at most 2^30
+// block rows.  A unit is 32 * bpt << unit_class blocks.
+struct ParamImage {
+    const uint8_t* src;
+    uint8_t* dst;
+    uint32_t stride;
+    uint32_t w;  // blocks per row, codec << 28, 16-byte aligned rows << 29, unit class bits 0-1 << 30
+    uint32_t h;  // block rows, unit class bits 2-3 << 30
+    uint32_t first_unit;
+
+    __host__ __device__ uint32_t bw() const { return w & 0x0fffffffu; }
+    __host__ __device__ uint32_t bh() const { return h & 0x3fffffffu; }
+    __host__ __device__ uint32_t codec() const { return w >> 28 & 1u; }
+    __host__ __device__ uint32_t vec16() const { return w >> 29 & 1u; }
+    __host__ __device__ uint32_t unit_class() const { return w >> 30 | h >> 30 << 2; }
+};
+static_assert(sizeof(ParamImage) == 32, "ParamImage layout");
+constexpr uint32_t kParamImages = 1022;
+
+// One launch of the work-unit kernel with its descriptors as the kernel's
+// parameter.  The launch copies 32, 256 or kParamImages entries, whichever
+// holds `count` (a smaller parameter launches faster): `images` has that room.
+struct ParamLaunch {
+    ParamImage* images;
+    uint32_t count, units;
+};
+cudaError_t launch_batch_params(const ParamLaunch& l, const BatchTile& tile, cudaStream_t stream);
+
 // Checks `count` caller images (codec, sizes multiples of 4, non-null and
 // aligned buffers, stride) and fills their device descriptors, the first-unit
 // table (`first[i]` = desc[i].first_unit) and the total of work units of
@@ -68,6 +99,10 @@ cudaError_t launch_batch_tma_inline(const InlineBatch& batch, uint32_t n_images,
 // status of the first bad image (with its message in the last error).
 int validate_and_fill(const goofy_gpu_image* images, uint32_t count, uint32_t unit_blocks, BatchImage* desc,
                       uint32_t* first, uint32_t* total_units);
+
+// The same checks into a parameter launch (count <= kParamImages): its table,
+// the size class of each image's units, their number.
+int validate_and_fill(const goofy_gpu_image* images, uint32_t count, const BatchTile& tile, ParamLaunch* l);
 
 // Enqueue the persistent batch kernel.  `work_counter` must read 0 when the
 // kernel starts; `first_unit[i]` is images[i].first_unit (ascending, [0] = 0).

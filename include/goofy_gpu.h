@@ -350,7 +350,9 @@ typedef struct goofy_gpu_batch goofy_gpu_batch;
 typedef struct goofy_gpu_batch_tile {
     uint32_t threads_per_cta;   /* 128, 256, 512 (compute threads; the pipeline adds a producer warp) */
     uint32_t blocks_per_thread; /* 1 or 2 */
-    uint32_t unit_blocks;       /* 4x4 blocks per work unit, a multiple of 32 * blocks_per_thread;
+    uint32_t unit_blocks;       /* 4x4 blocks per work unit, a multiple of 32 * blocks_per_thread
+                                 * (up to 2044 images: at most four times as many, fewer where
+                                 * that spreads the work further);
                                  * threads_per_cta * blocks_per_thread with pipeline = 1 */
     uint32_t pipeline;          /* 0: warps pull work units and load their rows themselves;
                                  * 1: per CTA a producer warp pulls units and bulk-copies their rows
@@ -366,10 +368,10 @@ void goofy_gpu_batch_destroy(goofy_gpu_batch* batch);
 /* Encode `count` images in one persistent launch: warps pull work units
  * (runs of unit_blocks blocks of one image) from a device work counter, or
  * with a pipeline tile each CTA's producer warp stages its units' rows in
- * shared memory.  Enqueued on `stream` (one descriptor upload and the
- * kernel, a CUDA graph replay for a repeated batch shape; with a pipeline
- * tile and at most 64 images, the descriptors are the kernel's parameter and
- * nothing is uploaded): ordered after the work already queued there, and
+ * shared memory.  Enqueued on `stream`: up to 2044 images (64 with a pipeline
+ * tile) as one or two launches that take the descriptors as their parameter,
+ * one unit a warp, and nothing is uploaded; more with one descriptor upload
+ * and the kernel, a CUDA graph replay for a repeated batch shape.  Ordered after the work already queued there, and
  * later work there waits for it.  Each image's output equals
  * goofy_gpu_compress_device on that image alone. */
 int goofy_gpu_batch_encode(goofy_gpu_batch* batch, const goofy_gpu_image* images, uint32_t count, void* stream);
@@ -496,21 +498,15 @@ int goofy_gpu_plain_replay(int device, const goofy_gpu_request* reqs, const int6
  * inside a renderer's frame budget, where the CUDA allocator can stall the
  * device, or an engine whose own allocator owns all GPU memory.  No
  * counterpart in the reference.
- * The work counter and descriptor tables live in one fixed file-scope device
- * array of the library (13,568 bytes, held on every GPU that loads the library
- * until the process exits), so a call takes at most GOOFY_NOALLOC_MAX_IMAGES
- * images; more returns GOOFY_ERR_TOO_LARGE, a NULL `images` with count > 0
- * GOOFY_ERR_INVALID, and an invalid image its status -- all before anything
- * is launched.  The caller's images (device src / dst) are the inputs and
- * outputs; they must be on the calling thread's current device, whose copy of
- * the array the call uses.  The first call in a context (a device's primary
- * context, again after cudaDeviceReset) looks up the array's device address
- * with cudaGetSymbolAddress; make that first call before any stream capture.
- * All calls share the array: calls whose GPU work overlaps (e.g. on two
- * unordered streams) race; issue them on one stream or order them.
- * Asynchronous on `stream`: two launches, a small kernel that takes the
- * call's tables as its parameter and writes them into the array, then the
- * batch kernel; no host memory is read after the call returns. */
+ * A call takes at most GOOFY_NOALLOC_MAX_IMAGES images; more returns
+ * GOOFY_ERR_TOO_LARGE, a NULL `images` with count > 0 GOOFY_ERR_INVALID, and
+ * an invalid image its status -- all before anything is launched.  The
+ * caller's images (device src / dst) are the inputs and outputs; they must be
+ * on the calling thread's current device.  The library holds no device memory
+ * for it and calls share nothing: they may run at the same time on any
+ * streams and be captured.
+ * Asynchronous on `stream`: one launch that takes the call's descriptors as
+ * its parameter; no host memory is read after the call returns. */
 int goofy_gpu_batch_encode_noalloc(const goofy_gpu_image* images, uint32_t count, void* stream);
 
 #ifdef __cplusplus

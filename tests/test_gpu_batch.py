@@ -265,3 +265,46 @@ def test_pipelined_batches_keep_stream_order(cuda, tile):
     want_b = oracle.encode(g.CODEC_ETC1S, other, w, h)
     np.testing.assert_array_equal(src[:n].cpu().numpy(), want_b)
     np.testing.assert_array_equal(r.cpu().numpy(), want_b)
+
+
+def _many(torch, n, seed, big=()):
+    """n small images (single blocks among them, some empty, some word-aligned) and `big` ones at the given places."""
+    rng = np.random.default_rng(seed)
+    items = []
+    for i in range(n):
+        w, h = dict(big).get(i) or (4 * int(rng.integers(0, 9)), 4 * int(rng.integers(1, 9)))
+        stride, offset = 4 * max(w, 4) + [0, 16, 4][i % 3], [0, 16, 4, 0][i % 4]
+        img = rng.integers(0, 256, (h, 4 * w), np.uint8)
+        rows = np.zeros((h, stride), np.uint8)
+        rows[:, :4 * w] = img
+        buf = np.zeros(h * stride + offset + 64, np.uint8)
+        buf[offset:offset + h * stride] = rows.reshape(-1)
+        k = g.out_size(w, h)
+        items.append(dict(src=torch.from_numpy(buf).cuda(), offset=offset, rows=rows, w=w, h=h, stride=stride,
+                          codec=i % 2, dst=torch.full((k + 2 * GUARD,), 0x5A, dtype=torch.uint8, device="cuda"), n=k))
+    return items
+
+
+@pytest.mark.parametrize("n", [1, 32, 33, 256, 257, 1022, 1023, 2044, 2045])
+def test_image_counts_around_the_parameter_tables(cuda, n):
+    """One launch up to 1022 images (tables of 32, 256, 1022), two up to 2044, an upload beyond."""
+    items = _many(cuda, n, n)
+    b = g.Batch(n)
+    try:
+        assert b.encode(descriptors(items), cuda.cuda.current_stream().cuda_stream) == g.OK, g.last_error()
+        check(cuda, items)
+    finally:
+        b.close()
+
+
+@pytest.mark.parametrize("tile", [(128, 1, 256, 0), (128, 2, 64, 0), (512, 1, 65536, 0), (256, 2, 192, 0)])
+def test_unit_sizes_fall_towards_the_end(cuda, tile):
+    """Large images first, small ones behind: units of every size class, down to one pass of a warp."""
+    items = _many(cuda, 40, 5, big=((0, (4096, 2052)), (3, (2052, 1024)), (9, (1028, 516)), (20, (4, 4096))))
+    b = g.Batch(len(items))
+    try:
+        assert b.set_tile(*tile) == g.OK
+        assert b.encode(descriptors(items), cuda.cuda.current_stream().cuda_stream) == g.OK, g.last_error()
+        check(cuda, items)
+    finally:
+        b.close()
