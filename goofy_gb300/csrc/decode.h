@@ -12,11 +12,27 @@ namespace goofy_gpu {
 cudaError_t launch_decode(int codec, const uint8_t* blocks, uint32_t width, uint32_t height, uint8_t* rgba,
                           size_t stride, unsigned long long* unsupported, cudaStream_t stream);
 
+// Where the sums go when the launch is their only user (`sums` and *finished
+// zero before it): the last CTA to finish writes the six totals to `host`
+// (mapped host memory) and leaves `sums` and *finished zero for the next.
+struct ErrorResult {
+    unsigned long long* host = nullptr;
+    unsigned int* finished = nullptr;
+};
+
 // Adds the per-channel sums of squared differences between `src` and the
 // decoded blocks to sums[0..3], the unsupported-block count to sums[4] and the
 // sum of squared luminosity differences (hundredths) to sums[5].
 cudaError_t launch_block_error(int codec, const uint8_t* blocks, const uint8_t* src, uint32_t width, uint32_t height,
-                               size_t stride, bool vec16, unsigned long long* sums, cudaStream_t stream);
+                               size_t stride, bool vec16, unsigned long long* sums, cudaStream_t stream,
+                               ErrorResult result = {});
+
+// The same on the bulk-copy ring (encode_tma.cu), images of 32 blocks a row and
+// more; `big`: CTAs of 512 threads x 2 blocks (rows of 205 blocks and more),
+// else 128 x 1.
+cudaError_t launch_error_tma(int codec, const uint8_t* blocks, const uint8_t* src, uint32_t width, uint32_t height,
+                             size_t stride, bool vec16, bool big, unsigned long long* sums, ErrorResult result,
+                             cudaStream_t stream);
 
 struct BatchImage;
 

@@ -7,10 +7,11 @@
 // differences in getMsePsnr (Src/main.cpp:403-469).  Here one thread decodes
 // one block (BC1: both endpoint orders; ETC1: individual and differential
 // modes, both flips; ETC2-only differential overflows are counted as
-// unsupported and decoded as black) and either stores the 16 pixels or
-// compares them with the source pixels, summing squared differences per
-// channel exactly in integers (64-bit per thread over a grid stride, then
-// shuffles and shared memory, one 64-bit atomic per CTA and channel).
+// unsupported and decoded as black) and either stores the 16 pixels or, in
+// the quality kernels, compares the block with its source pixels
+// (block_error.cuh), summing squared differences per channel exactly in
+// integers (32-bit per thread, then 64-bit through shuffles and shared memory,
+// one atomic per CTA and sum).
 #include <cuda_runtime.h>
 
 #include <atomic>
@@ -18,8 +19,10 @@
 #include "batch.h"
 #include "block_codec.cuh"
 #include "block_decode.cuh"
+#include "block_error.cuh"
 #include "decode.h"
 #include "device_io.cuh"
+#include "error_reduce.cuh"
 #include "pdl.cuh"
 
 namespace goofy_gpu {
@@ -27,13 +30,6 @@ namespace goofy_gpu {
 // Threads per CTA of every decoding kernel: the palette column stride, a
 // constant so that a pixel's palette address is a shift and an add.
 constexpr uint32_t kDecodeThreads = 256;
-
-__device__ __forceinline__ uint2 load_block8(const uint8_t* p)
-{
-    uint2 v;
-    asm("ld.global.nc.L1::no_allocate.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
-    return v;
-}
 
 template <int CODEC>
 __global__ void __launch_bounds__(kDecodeThreads) decode_image_kernel(const uint8_t* __restrict__ blocks, uint32_t bw,
@@ -59,67 +55,23 @@ __global__ void __launch_bounds__(kDecodeThreads) decode_image_kernel(const uint
     if (bad && (threadIdx.x & 31u) == 0) atomicAdd(unsupported, (unsigned long long)__popc(bad));
 }
 
-// Sums of squared channel differences of one 4-pixel row: |a-b| per byte,
-// bytes regrouped so each word holds one channel of the 4 pixels, then a
-// dot product of each channel word with itself.
-__device__ __forceinline__ void accumulate_row(const uint32_t (&a)[4], const uint32_t (&b)[4], uint32_t (&acc)[4])
-{
-    uint32_t d[4];
-#pragma unroll
-    for (int x = 0; x < 4; ++x) d[x] = __vabsdiffu4(a[x], b[x]);
-    const uint32_t t0 = __byte_perm(d[0], d[1], 0x5140), t1 = __byte_perm(d[2], d[3], 0x5140);
-    const uint32_t t2 = __byte_perm(d[0], d[1], 0x7362), t3 = __byte_perm(d[2], d[3], 0x7362);
-    const uint32_t ch[4] = {__byte_perm(t0, t1, 0x5410), __byte_perm(t0, t1, 0x7632), __byte_perm(t2, t3, 0x5410),
-                            __byte_perm(t2, t3, 0x7632)};
-#pragma unroll
-    for (int c = 0; c < 4; ++c) acc[c] = __dp4a(ch[c], ch[c], acc[c]);
-}
-
-// The harness's luminosity difference (0.21 R + 0.72 G + 0.07 B of a pixel
-// read as a little-endian u32, R = byte 2) in hundredths, which is exact in
-// integers: 21 * d(byte 2) + 72 * d(byte 1) + 7 * d(byte 0).  Two byte dot
-// products: the second multiplies b's unsigned bytes by the negated weights
-// (signed bytes) and adds the first, so no subtraction is needed.
-__device__ __forceinline__ int luma_diff(uint32_t a, uint32_t b)
-{
-    constexpr uint32_t kWeights = 0x00154807u;     // bytes 0..3: 7, 72, 21, 0
-    constexpr uint32_t kNegWeights = 0x00ebb8f9u;  // bytes 0..3: -7, -72, -21, 0
-    int d;
-    asm("dp4a.u32.s32 %0, %1, %2, %3;" : "=r"(d) : "r"(b), "r"(kNegWeights), "r"((int)__dp4a(a, kWeights, 0u)));
-    return d;
-}
-
-// Squared luminosity differences summed over a row of 4 pixels (at most
-// 4 * 25500^2 < 2^32).
-__device__ __forceinline__ uint32_t luma_row(const uint32_t (&a)[4], const uint32_t (&b)[4])
-{
-    uint32_t acc = 0;
-#pragma unroll
-    for (int x = 0; x < 4; ++x) {
-        const int d = luma_diff(a[x], b[x]);
-        acc += (uint32_t)(d * d);
-    }
-    return acc;
-}
-
-// Resident grid: each thread walks blocks with a grid stride, keeps 64-bit
-// sums, then the CTA reduces (shuffles, shared memory) and adds its six
-// totals with one atomic each.  Register caps for 4 (BC1, 64 registers) /
-// 3 (ETC1, 80) CTAs per SM, no spills: uncapped, ETC1 took 94 registers and
-// 2 CTAs per SM (51.3 against 47.4 us at 8192^2); capped at 4 CTAs it
-// spilled (50.9 us).
+// Tiny images and narrow rows; the others take error_image_tma (encode_tma.cu).
+// Resident grid: each thread walks blocks with a grid stride, then the CTA
+// reduces and adds its six totals.  Register caps for 4 (BC1) / 3 (ETC1) CTAs
+// per SM, no spills.
 template <int CODEC>
 __global__ void __launch_bounds__(kDecodeThreads, CODEC == kBC1 ? 4 : 3)
     block_error_kernel(const uint8_t* __restrict__ blocks, uint32_t bw, uint32_t nblk, const uint8_t* __restrict__ src,
-                       size_t stride, bool vec16, unsigned long long* __restrict__ sums)
+                       size_t stride, bool vec16, unsigned long long* __restrict__ sums, ErrorResult result)
 {
     pdl_launch_dependents();
-    __shared__ uint32_t pal[8 * kDecodeThreads];
-    unsigned long long s[6] = {0, 0, 0, 0, 0, 0};
+    __shared__ uint32_t pal[CODEC == kBC1 ? 1 : 8 * kDecodeThreads];  // for ETC1 blocks of other shapes than ETC1s
     const uint32_t bw_magic = 0xffffffffu / bw;
+    ErrorSums e{};  // at most kErrorSumBlocks blocks a thread (launch_block_error)
+    uint32_t bad = 0;
     pdl_wait();
     // software pipeline: the next block's source rows and code are loaded
-    // before this block is decoded and compared
+    // before this block is compared
     const uint32_t step = gridDim.x * kDecodeThreads;
     uint32_t i = blockIdx.x * kDecodeThreads + threadIdx.x;
     uint32_t w[16];
@@ -131,7 +83,7 @@ __global__ void __launch_bounds__(kDecodeThreads, CODEC == kBC1 ? 4 : 3)
         blk = load_block8(blocks + 8u * (size_t)i);
     }
     for (; i < nblk; i += step) {
-        uint32_t px[16], cur[16];
+        uint32_t cur[16];
 #pragma unroll
         for (int k = 0; k < 16; ++k) cur[k] = w[k];
         const uint2 cur_blk = blk;
@@ -141,33 +93,11 @@ __global__ void __launch_bounds__(kDecodeThreads, CODEC == kBC1 ? 4 : 3)
             load_block_rows(src + (size_t)by * 4u * stride + 16u * (size_t)bx, stride, vec16, w);
             blk = load_block8(blocks + 8u * (size_t)(i + step));
         }
-        const bool ok = decode_block<CODEC>(cur_blk, pal + threadIdx.x, kDecodeThreads, px);
-        uint32_t acc[4] = {0, 0, 0, 0};  // one block: at most 16 * 255^2 per channel
-#pragma unroll
-        for (int y = 0; y < 4; ++y) {
-            const uint32_t a[4] = {cur[4 * y], cur[4 * y + 1], cur[4 * y + 2], cur[4 * y + 3]};
-            const uint32_t b[4] = {px[4 * y], px[4 * y + 1], px[4 * y + 2], px[4 * y + 3]};
-            accumulate_row(a, b, acc);
-            s[5] += luma_row(a, b);
-        }
-#pragma unroll
-        for (int c = 0; c < 4; ++c) s[c] += acc[c];
-        s[4] += ok ? 0u : 1u;
+        if (!add_block_errors<CODEC>(cur, cur_blk, pal + threadIdx.x, kDecodeThreads, e)) ++bad;
     }
-    __shared__ unsigned long long part[6][8];
-    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-#pragma unroll
-    for (int c = 0; c < 6; ++c) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) s[c] += __shfl_xor_sync(0xffffffffu, s[c], o);
-        if (lane == 0) part[c][warp] = s[c];
-    }
-    __syncthreads();
-    if (threadIdx.x < 6) {
-        unsigned long long t = 0;
-        for (uint32_t k = 0; k < (kDecodeThreads >> 5); ++k) t += part[threadIdx.x][k];
-        if (t) atomicAdd(&sums[threadIdx.x], t);
-    }
+    __shared__ unsigned long long part[6][kDecodeThreads / 32];
+    const uint64_t s[6] = {e.sq[0], e.sq[1], e.sq[2], e.sq[3], bad, luma_sum_of(e)};
+    reduce_errors<kDecodeThreads>(s, part, sums, result);
 }
 
 // The error sums of every image of a batch (the request server's quality
@@ -191,27 +121,20 @@ __global__ void __launch_bounds__(kDecodeThreads) quality_batch_kernel(const Bat
         const uint32_t ii = find_image(first_unit, n_images, u);
         const BatchImage im = images[ii];
         const uint32_t first = (u - im.first_unit) * unit_blocks, last = min(first + unit_blocks, im.bw * im.bh);
-        // per lane at most 2048 blocks of a unit: 2048 * 16 * 255^2 < 2^32 per channel
-        uint32_t acc[4] = {0, 0, 0, 0}, bad = 0;
-        unsigned long long ys = 0;
+        ErrorSums e{};  // a lane has at most kErrorSumBlocks blocks of a unit (launch_quality_batch)
+        uint32_t bad = 0;
         for (uint32_t b = first + lane; b < last; b += 32u) {
             uint32_t bx;
             const uint32_t by = div_magic(b, im.bw, im.bw_magic, bx);
-            uint32_t px[16], w[16];
+            uint32_t w[16];
             const uint2 blk = load_block8(im.dst + 8u * (size_t)b);
-            const bool ok = im.codec == kBC1 ? decode_block<kBC1>(blk, pal + threadIdx.x, kDecodeThreads, px)
-                                             : decode_block<kETC1S>(blk, pal + threadIdx.x, kDecodeThreads, px);
             load_block_rows(im.src + (size_t)by * 4u * im.stride + 16u * (size_t)bx, im.stride, im.vec16 != 0, w);
-#pragma unroll
-            for (int y = 0; y < 4; ++y) {
-                const uint32_t a[4] = {w[4 * y], w[4 * y + 1], w[4 * y + 2], w[4 * y + 3]};
-                const uint32_t d[4] = {px[4 * y], px[4 * y + 1], px[4 * y + 2], px[4 * y + 3]};
-                accumulate_row(a, d, acc);
-                ys += luma_row(a, d);
-            }
+            const bool ok = im.codec == kBC1
+                                ? add_block_errors<kBC1>(w, blk, pal + threadIdx.x, kDecodeThreads, e)
+                                : add_block_errors<kETC1S>(w, blk, pal + threadIdx.x, kDecodeThreads, e);
             bad += ok ? 0u : 1u;
         }
-        unsigned long long t[6] = {acc[0], acc[1], acc[2], acc[3], bad, ys};
+        unsigned long long t[6] = {e.sq[0], e.sq[1], e.sq[2], e.sq[3], bad, luma_sum_of(e)};
 #pragma unroll
         for (int c = 0; c < 6; ++c) {
 #pragma unroll
@@ -229,6 +152,7 @@ cudaError_t launch_quality_batch(const BatchImage* images, uint32_t n_images, co
                                  unsigned long long* sums, cudaStream_t stream)
 {
     if (total_units == 0) return cudaSuccess;
+    if (unit_blocks > 32u * kErrorSumBlocks) return cudaErrorInvalidValue;
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -277,25 +201,33 @@ uint32_t resident_per_sm(K kernel, int dev, int slot)
 }  // namespace
 
 cudaError_t launch_block_error(int codec, const uint8_t* blocks, const uint8_t* src, uint32_t width, uint32_t height,
-                               size_t stride, bool vec16, unsigned long long* sums, cudaStream_t stream)
+                               size_t stride, bool vec16, unsigned long long* sums, cudaStream_t stream,
+                               ErrorResult result)
 {
     const uint32_t bw = width / 4, nblk = bw * (height / 4);
     if (nblk == 0) return cudaSuccess;
+    // The lines are the image encoder's (launch_image).  Launches back to back (us), this kernel / the ring, BC1
+    // and ETC1s: 2048^2 6.1 / 5.1 and 5.9 / 5.1, 4096^2 14.1 / 12.9 and 14.0 / 12.8, 8192^2 46.0 / 42.7 and 46.7 /
+    // 42.7 (floors 2.8, 11.3, 45.1 at 4.5 B/px of measured HBM: nothing is written, and reads alone run faster than
+    // the copy the floor is taken from); 1024^2 2.8 / 3.1 with the image in L2, 3.7 / 3.3 from HBM.
+    if (nblk >= 20000 && bw >= 32)
+        return launch_error_tma(codec, blocks, src, width, height, stride, vec16, nblk >= 600000 && bw >= 256, sums,
+                                result, stream);
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     // One wave: as many CTAs as fit on the GPU at once, each thread striding
-    // over its share of the blocks.  A grid of 8 CTAs per SM ran in 2.7
-    // waves for BC1 and left SMs part-empty in the last one (50.6 against
-    // 47.2 us at 8192^2).
+    // over its share of the blocks (more for an image so long and narrow that
+    // a thread's 32-bit sums would run over).
     const uint32_t per_sm = codec == kBC1 ? resident_per_sm(block_error_kernel<kBC1>, dev, 0)
                                           : resident_per_sm(block_error_kernel<kETC1S>, dev, 1);
-    const uint32_t grid = min((nblk + kDecodeThreads - 1) / kDecodeThreads, (uint32_t)(sms > 0 ? sms : 1) * per_sm);
+    const uint32_t most = (nblk + kDecodeThreads - 1) / kDecodeThreads, least = (most + kErrorSumBlocks - 1) / kErrorSumBlocks;
+    const uint32_t grid = max(least, min(most, (uint32_t)(sms > 0 ? sms : 1) * per_sm));
     if (codec == kBC1)
         return launch_pdl(block_error_kernel<kBC1>, dim3(grid), dim3(kDecodeThreads), 0, stream, blocks, bw, nblk, src, stride,
-                          vec16, sums);
+                          vec16, sums, result);
     return launch_pdl(block_error_kernel<kETC1S>, dim3(grid), dim3(kDecodeThreads), 0, stream, blocks, bw, nblk, src, stride,
-                      vec16, sums);
+                      vec16, sums, result);
 }
 
 }  // namespace goofy_gpu

@@ -23,6 +23,14 @@ __device__ __forceinline__ uint32_t ld_once4(const uint8_t* p)
     return v;
 }
 
+// An encoded block.
+__device__ __forceinline__ uint2 load_block8(const uint8_t* p)
+{
+    uint2 v;
+    asm("ld.global.nc.L1::no_allocate.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
+    return v;
+}
+
 // Encoded blocks are written once and not read back by the kernel: streaming store.
 __device__ __forceinline__ void st_stream8(uint8_t* p, uint2 v)
 {

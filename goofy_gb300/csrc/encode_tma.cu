@@ -40,12 +40,16 @@
 // producer then waits (bounded) for the copies it issued before its CTA exits.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <atomic>
 
 #include "async_copy.cuh"
 #include "batch.h"
 #include "block_codec.cuh"
+#include "block_error.cuh"
+#include "decode.h"
 #include "device_io.cuh"
+#include "error_reduce.cuh"
 #include "kernels.h"
 #include "pdl.cuh"
 
@@ -120,13 +124,11 @@ __host__ __device__ constexpr uint32_t l2_prefetch_tiles(const TmaLayout& l)
 // (four lanes a bank, 64 wavefronts a warp and block instead of 16, which the
 // load/store unit has room for; picking the words out of two 16-byte loads
 // would take 36 selects a block on the busy ALU pipe).
-template <int CODEC, int BPT, bool WORD>
-__device__ __forceinline__ void encode_stage(const uint8_t* buf, uint32_t row_bytes, uint32_t warp, uint32_t lane,
-                                             uint32_t nb, uint8_t* out, uint8_t* out2, const uint8_t* ctrl_lut,
-                                             uint32_t bx0, uint32_t bw, uint32_t bw_magic,
-                                             const uint32_t (&shift)[4])
+template <int BPT, bool WORD>
+__device__ __forceinline__ void load_stage(const uint8_t* buf, uint32_t row_bytes, uint32_t warp, uint32_t lane,
+                                           uint32_t nb, uint32_t bx0, uint32_t bw, uint32_t bw_magic,
+                                           const uint32_t (&shift)[4], uint32_t (&w)[BPT][16])
 {
-    uint32_t w[BPT][16];
 #pragma unroll
     for (int j = 0; j < BPT; ++j) {
         const uint32_t b = (warp * BPT + j) * 32u + lane;
@@ -150,6 +152,16 @@ __device__ __forceinline__ void encode_stage(const uint8_t* buf, uint32_t row_by
             }
         }
     }
+}
+
+template <int CODEC, int BPT, bool WORD>
+__device__ __forceinline__ void encode_stage(const uint8_t* buf, uint32_t row_bytes, uint32_t warp, uint32_t lane,
+                                             uint32_t nb, uint8_t* out, uint8_t* out2, const uint8_t* ctrl_lut,
+                                             uint32_t bx0, uint32_t bw, uint32_t bw_magic,
+                                             const uint32_t (&shift)[4])
+{
+    uint32_t w[BPT][16];
+    load_stage<BPT, WORD>(buf, row_bytes, warp, lane, nb, bx0, bw, bw_magic, shift, w);
 #pragma unroll
     for (int j = 0; j < BPT; ++j) {
         const uint32_t b = (warp * BPT + j) * 32u + lane;
@@ -186,11 +198,111 @@ __device__ __forceinline__ void for_unit_rows(const uint8_t* src, size_t stride,
     }
 }
 
-// WORD: the rows are only 4-byte aligned.  4 * stride is then a multiple of
-// 16, so pixel row y of every block row starts shift[y] = (src + y * stride)
-// % 16 bytes past a 16-byte boundary; the copies take whole granules from that
-// boundary on (the first and last may hold bytes of other pixels, never of
-// another allocation's page) and the compute warps read at the shift.
+// The image behind a ring.  WORD: its rows are only 4-byte aligned.
+// 4 * stride is then a multiple of 16, so pixel row y of every block row
+// starts shift[y] = (src + y * stride) % 16 bytes past a 16-byte boundary; the
+// copies take whole granules from that boundary on (the first and last may
+// hold bytes of other pixels, never of another allocation's page) and the
+// compute warps read at the shift.
+template <bool WORD>
+struct RingImage {
+    const uint8_t* src;
+    size_t stride;
+    uint32_t bw, bw_magic, total;
+    uint32_t shift[4];
+
+    __device__ __forceinline__ RingImage(const uint8_t* src_, size_t stride_, uint32_t bw_, uint32_t magic, uint32_t n)
+        : src(src_), stride(stride_), bw(bw_), bw_magic(magic), total(n)
+    {
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+            shift[r] = WORD ? (uint32_t)(reinterpret_cast<uintptr_t>(src) + r * stride) & 15u : 0u;
+    }
+
+    // bytes of pixel row r's piece of nb blocks
+    __device__ __forceinline__ uint32_t piece(uint32_t nb, int r) const
+    {
+        return WORD ? (16u * nb + shift[r] + 15u) & ~15u : 16u * nb;
+    }
+};
+
+// One lane, before the dependency wait: while the previous kernel in the
+// stream drains, ask L2 for the rows of this CTA's first units.  Only a hint:
+// no data enters the CTA before pdl_wait(), and L2 is coherent with the
+// previous kernel's writes, so the copies after the wait still read what it
+// wrote.
+template <bool WORD>
+__device__ __forceinline__ void prefetch_units(const RingImage<WORD>& im, const TmaLayout& L)
+{
+    const uint32_t unit = L.tile_blocks, step = gridDim.x * unit;
+    uint32_t c = 0;
+    for (uint32_t first = blockIdx.x * unit; first < im.total && c < l2_prefetch_tiles(L); first += step, ++c)
+        for_unit_rows(im.src, im.stride, im.bw, im.bw_magic, first, min(unit, im.total - first),
+                      [&](uint32_t, uint32_t nb, const uint8_t* row) {
+#pragma unroll
+                          for (int r = 0; r < 4; ++r)
+                              bulk_prefetch_l2(row + r * im.stride - im.shift[r], im.piece(nb, r));
+                      });
+}
+
+// The producer's one lane: copies the rows of units blockIdx.x, + gridDim.x,
+// ... into the ring, each stage once its compute warps have released it.
+template <bool WORD>
+__device__ __forceinline__ void produce_units(const RingImage<WORD>& im, const TmaLayout& L, uint8_t* smem,
+                                              uint64_t* full, uint64_t* empty, volatile uint32_t* abort_flag,
+                                              uint64_t policy)
+{
+    const uint32_t unit = L.tile_blocks, step = gridDim.x * unit;
+    uint32_t issued = 0, slot = 0, phase = 0;
+    for (uint32_t first = blockIdx.x * unit; first < im.total; first += step) {
+        if (issued >= L.stages && !mbar_wait(&empty[slot], phase ^ 1u, abort_flag, &g_pipeline_timeouts)) break;
+        const uint32_t n = min(unit, im.total - first);
+        uint32_t bytes = 64u * n, s = 0;
+        if constexpr (WORD) {
+            bytes = 0;
+            for_unit_rows(im.src, im.stride, im.bw, im.bw_magic, first, n,
+                          [&](uint32_t, uint32_t nb, const uint8_t*) {
+#pragma unroll
+                              for (int r = 0; r < 4; ++r) bytes += im.piece(nb, r);
+                          });
+        }
+        mbar_arrive_expect_tx(&full[slot], bytes);
+        uint8_t* buf = smem + slot * L.stage_bytes;
+        for_unit_rows(im.src, im.stride, im.bw, im.bw_magic, first, n,
+                      [&](uint32_t k, uint32_t nb, const uint8_t* row) {
+#pragma unroll
+                          for (int r = 0; r < 4; ++r)
+                              bulk_copy_g2s_hint(buf + r * L.row_bytes + 16u * (k + s),
+                                                 row + r * im.stride - im.shift[r], im.piece(nb, r), &full[slot],
+                                                 policy);
+                          if constexpr (WORD) ++s;
+                      });
+        ++issued;
+        if (++slot == L.stages) {
+            slot = 0;
+            phase ^= 1u;
+        }
+    }
+    if (*abort_flag) {
+        // the copies of the last stages may still be landing: wait for them (bounded) before exiting
+        const uint32_t n = issued < L.stages ? issued : L.stages;
+        for (uint32_t i = issued - n; i < issued; ++i)
+            mbar_wait(&full[i % L.stages], (i / L.stages) & 1u, nullptr, &g_pipeline_timeouts);
+    }
+}
+
+// One thread, at a CTA's start.
+__device__ __forceinline__ void init_ring(uint64_t* full, uint64_t* empty, uint32_t stages, uint32_t compute_warps,
+                                          uint32_t* abort_flag)
+{
+    for (uint32_t s = 0; s < stages; ++s) {
+        mbar_init(&full[s], 1u);
+        mbar_init(&empty[s], compute_warps);
+    }
+    *abort_flag = 0u;
+    mbar_init_fence();
+}
+
 template <int CODEC, int BPT, int COMPUTE, bool WORD>
 __global__ void __launch_bounds__(COMPUTE + 32, tma_min_ctas(BPT, COMPUTE))
     encode_image_tma(const uint8_t* __restrict__ src, size_t stride, uint8_t* __restrict__ dst,
@@ -205,83 +317,27 @@ __global__ void __launch_bounds__(COMPUTE + 32, tma_min_ctas(BPT, COMPUTE))
     uint64_t* empty = full + L.stages;
     uint8_t* ctrl_lut = reinterpret_cast<uint8_t*>(empty + L.stages);
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
-    constexpr uint32_t unit = L.tile_blocks;
-    const uint32_t step = gridDim.x * unit;  // units blockIdx.x, + gridDim.x, ...
-    uint32_t shift[4];
-#pragma unroll
-    for (int r = 0; r < 4; ++r) shift[r] = WORD ? (uint32_t)(reinterpret_cast<uintptr_t>(src) + r * stride) & 15u : 0u;
-    // bytes of pixel row r's piece of nb blocks
-    auto piece = [&](uint32_t nb, int r) { return WORD ? (16u * nb + shift[r] + 15u) & ~15u : 16u * nb; };
+    const RingImage<WORD> im(src, stride, bw, bw_magic, total);
 
-    if (threadIdx.x == 0) {
-        for (uint32_t s = 0; s < L.stages; ++s) {
-            mbar_init(&full[s], 1u);
-            mbar_init(&empty[s], compute_warps);
-        }
-        abort_flag = 0u;
-        mbar_init_fence();
-    }
+    if (threadIdx.x == 0) init_ring(full, empty, L.stages, compute_warps, &abort_flag);
     if constexpr (CODEC != kBC1) fill_ctrl_lut(ctrl_lut);
     __syncthreads();
-    if (warp == compute_warps && lane == 0) {
-        // While the previous kernel in the stream drains, ask L2 for the rows
-        // of this CTA's first units.  Only a hint: no data enters the CTA
-        // before pdl_wait(), and L2 is coherent with the previous kernel's
-        // writes, so the copies after the wait still read what it wrote.
-        uint32_t c = 0;
-        for (uint32_t first = blockIdx.x * unit; first < total && c < l2_prefetch_tiles(L); first += step, ++c)
-            for_unit_rows(src, stride, bw, bw_magic, first, min(unit, total - first),
-                          [&](uint32_t, uint32_t nb, const uint8_t* row) {
-#pragma unroll
-                              for (int r = 0; r < 4; ++r) bulk_prefetch_l2(row + r * stride - shift[r], piece(nb, r));
-                          });
-    }
+    if (warp == compute_warps && lane == 0) prefetch_units(im, L);
     pdl_wait();  // no global memory access before the previous kernel in the stream is done
 
     if (warp == compute_warps) {  // producer
-        if (lane != 0) return;
         // Rows are read once: evict-first in L2 (single-codec launches back to
         // back: 4096^2 ETC1s 12.3 against 13.2 us, BC1 11.2 against 12.4 us).
         // The two-codec pass marks half of them: with all it measured 0.9 us
         // slower at 8192^2; with half, as fast there and 0.4 us faster at 4096^2.
-        const uint64_t policy = CODEC == kBoth ? l2_evict_first_half_policy() : l2_evict_first_policy();
-        uint32_t issued = 0, slot = 0, phase = 0;
-        for (uint32_t first = blockIdx.x * unit; first < total; first += step) {
-            if (issued >= L.stages && !mbar_wait(&empty[slot], phase ^ 1u, &abort_flag, &g_pipeline_timeouts))
-                break;
-            const uint32_t n = min(unit, total - first);
-            uint32_t bytes = 64u * n, s = 0;
-            if constexpr (WORD) {
-                bytes = 0;
-                for_unit_rows(src, stride, bw, bw_magic, first, n, [&](uint32_t, uint32_t nb, const uint8_t*) {
-#pragma unroll
-                    for (int r = 0; r < 4; ++r) bytes += piece(nb, r);
-                });
-            }
-            mbar_arrive_expect_tx(&full[slot], bytes);
-            uint8_t* buf = smem + slot * L.stage_bytes;
-            for_unit_rows(src, stride, bw, bw_magic, first, n, [&](uint32_t k, uint32_t nb, const uint8_t* row) {
-#pragma unroll
-                for (int r = 0; r < 4; ++r)
-                    bulk_copy_g2s_hint(buf + r * L.row_bytes + 16u * (k + s), row + r * stride - shift[r],
-                                       piece(nb, r), &full[slot], policy);
-                if constexpr (WORD) ++s;
-            });
-            ++issued;
-            if (++slot == L.stages) {
-                slot = 0;
-                phase ^= 1u;
-            }
-        }
-        if (*static_cast<volatile uint32_t*>(&abort_flag)) {
-            // the copies of the last stages may still be landing: wait for them (bounded) before exiting
-            const uint32_t n = issued < L.stages ? issued : L.stages;
-            for (uint32_t i = issued - n; i < issued; ++i)
-                mbar_wait(&full[i % L.stages], (i / L.stages) & 1u, nullptr, &g_pipeline_timeouts);
-        }
+        if (lane == 0)
+            produce_units(im, L, smem, full, empty, &abort_flag,
+                          CODEC == kBoth ? l2_evict_first_half_policy() : l2_evict_first_policy());
         return;
     }
 
+    constexpr uint32_t unit = L.tile_blocks;
+    const uint32_t step = gridDim.x * unit;  // units blockIdx.x, + gridDim.x, ...
     uint32_t slot = 0, phase = 0;
     for (uint32_t first = blockIdx.x * unit; first < total; first += step) {
         if (!mbar_wait(&full[slot], phase, &abort_flag, &g_pipeline_timeouts)) break;
@@ -292,7 +348,7 @@ __global__ void __launch_bounds__(COMPUTE + 32, tma_min_ctas(BPT, COMPUTE))
         if constexpr (WORD) div_magic(first, bw, bw_magic, bx0);
         if (warp * (BPT * 32u) < nb)  // warps wholly past the unit's last block skip it
             encode_stage<CODEC, BPT, WORD>(buf, L.row_bytes, warp, lane, nb, dst + o,
-                                           CODEC == kBoth ? dst2 + o : nullptr, ctrl_lut, bx0, bw, bw_magic, shift);
+                                           CODEC == kBoth ? dst2 + o : nullptr, ctrl_lut, bx0, bw, bw_magic, im.shift);
         // Release the stage only now.  An arrival right after the shared loads
         // can overtake them: the loads wait in the load/store queue (behind
         // other kernels' global loads when SMs are shared) while the arrival
@@ -310,6 +366,82 @@ __global__ void __launch_bounds__(COMPUTE + 32, tma_min_ctas(BPT, COMPUTE))
     }
 }
 
+
+// ---------------------------------------------------------------------------
+// The quality measurement on the same ring: the compute warps compare each
+// block with its rows (block_error.cuh) instead of encoding it.  A thread's
+// codes of the next unit are loaded while it works on this one.  Bound by
+// HBM at 8192^2 (42.7 us, 7.07 TB/s); with the rows loaded into registers a
+// block ahead it was short of bytes in flight (46.0 us, and 14.1 against 12.9
+// at 4096^2).  The arithmetic alone did not change that: the same sums from
+// pixels decoded through shared memory took as long.
+// ---------------------------------------------------------------------------
+template <int CODEC, int BPT, int COMPUTE, bool WORD>
+__global__ void __launch_bounds__(COMPUTE + 32, BPT == 2 ? 1 : CODEC == kBC1 ? 6 : 5)
+    error_image_tma(const uint8_t* __restrict__ blocks, const uint8_t* __restrict__ src, size_t stride, uint32_t bw,
+                    uint32_t bw_magic, uint32_t total, unsigned long long* __restrict__ sums, ErrorResult result)
+{
+    pdl_launch_dependents();
+    extern __shared__ __align__(128) uint8_t smem[];
+    __shared__ uint32_t abort_flag;
+    constexpr uint32_t compute_warps = COMPUTE / 32;
+    constexpr TmaLayout L = tma_layout(COMPUTE, BPT, WORD);
+    uint64_t* full = reinterpret_cast<uint64_t*>(smem + L.stages * L.stage_bytes);
+    uint64_t* empty = full + L.stages;
+    uint32_t* pal = reinterpret_cast<uint32_t*>(empty + L.stages);  // ETC1 blocks of other shapes than ETC1s
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+    const RingImage<WORD> im(src, stride, bw, bw_magic, total);
+
+    if (threadIdx.x == 0) init_ring(full, empty, L.stages, compute_warps, &abort_flag);
+    __syncthreads();
+    if (warp == compute_warps && lane == 0) prefetch_units(im, L);
+    pdl_wait();
+
+    if (warp == compute_warps) {
+        if (lane == 0) produce_units(im, L, smem, full, empty, &abort_flag, l2_evict_first_policy());
+        return;
+    }
+
+    constexpr uint32_t unit = L.tile_blocks;
+    const uint32_t step = gridDim.x * unit;
+    uint32_t first = blockIdx.x * unit, slot = 0, phase = 0, bad = 0;
+    ErrorSums e{};  // at most kErrorSumBlocks blocks a thread (launch_error_tma)
+    uint2 next[BPT];
+    auto load_codes = [&](uint32_t at) {
+#pragma unroll
+        for (int j = 0; j < BPT; ++j) {
+            const uint32_t b = at + (warp * BPT + j) * 32u + lane;
+            next[j] = b < total ? load_block8(blocks + 8u * (size_t)b) : make_uint2(0u, 0u);
+        }
+    };
+    if (first < total) load_codes(first);
+    for (; first < total; first += step) {
+        uint2 code[BPT];
+#pragma unroll
+        for (int j = 0; j < BPT; ++j) code[j] = next[j];
+        if (first + step < total) load_codes(first + step);
+        if (!mbar_wait(&full[slot], phase, &abort_flag, &g_pipeline_timeouts)) break;
+        const uint32_t nb = min(unit, total - first);
+        uint32_t bx0 = 0, w[BPT][16];
+        if constexpr (WORD) div_magic(first, bw, bw_magic, bx0);
+        load_stage<BPT, WORD>(smem + slot * L.stage_bytes, L.row_bytes, warp, lane, nb, bx0, bw, bw_magic, im.shift, w);
+#pragma unroll
+        for (int j = 0; j < BPT; ++j)
+            if ((warp * BPT + j) * 32u + lane < nb)
+                bad += add_block_errors<CODEC>(w[j], code[j], pal + threadIdx.x, COMPUTE, e) ? 0u : 1u;
+        // Release the stage only now (see encode_image_tma): every loaded word has gone into these sums.
+        asm volatile("" ::"r"(e.sq[0]), "r"(e.sq[1]), "r"(e.sq[2]), "r"(e.sq[3]) : "memory");
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&empty[slot]);
+        if (++slot == L.stages) {
+            slot = 0;
+            phase ^= 1u;
+        }
+    }
+    __shared__ unsigned long long part[6][compute_warps];
+    const uint64_t s[6] = {e.sq[0], e.sq[1], e.sq[2], e.sq[3], bad, luma_sum_of(e)};
+    reduce_errors<COMPUTE>(s, part, sums, result);
+}
 
 // ---------------------------------------------------------------------------
 // The batch kernel on the same pipeline (tile `pipeline` = 1).  A work unit is
@@ -357,14 +489,7 @@ __device__ __forceinline__ void batch_tma_body(const BatchImage* __restrict__ im
     uint8_t* ctrl_lut = reinterpret_cast<uint8_t*>(rec + L.stages);
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
 
-    if (threadIdx.x == 0) {
-        for (uint32_t s = 0; s < L.stages; ++s) {
-            mbar_init(&full[s], 1u);
-            mbar_init(&empty[s], compute_warps);
-        }
-        abort_flag = 0u;
-        mbar_init_fence();
-    }
+    if (threadIdx.x == 0) init_ring(full, empty, L.stages, compute_warps, &abort_flag);
     fill_ctrl_lut(ctrl_lut);
     __syncthreads();
     if constexpr (PARAM_TABLES) {
@@ -537,41 +662,47 @@ __global__ void __launch_bounds__(COMPUTE + 32, tma_min_ctas(BPT, COMPUTE))
 
 namespace {
 
-template <int CODEC, int BPT, int COMPUTE, bool WORD>
-cudaError_t launch_tma_t(const uint8_t* src, size_t stride, uint8_t* dst, uint8_t* dst2, uint32_t bw, uint32_t bh,
-                         cudaStream_t stream)
+// Resident CTAs of a ring kernel on the current device, kept per device in
+// `resident`; the first call opts in to its shared memory.
+template <typename K>
+cudaError_t resident_ctas_of(K kernel, uint32_t threads, size_t smem, std::atomic<int> (&resident)[64], int* out)
 {
-    constexpr TmaLayout L = tma_layout(COMPUTE, BPT, WORD);
-    const size_t smem = tma_smem_bytes(L);
-    constexpr uint32_t block = COMPUTE + 32u;
-    // per device: dynamic shared memory opt-in and resident CTAs per SM
-    static std::atomic<int> resident[64];
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
     if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
     int ctas = resident[dev].load(std::memory_order_relaxed);
     if (ctas == 0) {
-        e = cudaFuncSetAttribute(encode_image_tma<CODEC, BPT, COMPUTE, WORD>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)smem);
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
-        e = cudaFuncSetAttribute(encode_image_tma<CODEC, BPT, COMPUTE, WORD>,
-                                 cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
         if (e != cudaSuccess) return e;
         int sms = 0, per_sm = 0;
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, encode_image_tma<CODEC, BPT, COMPUTE, WORD>, (int)block,
-                                                          smem);
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, (int)threads, smem);
         if (e != cudaSuccess) return e;
         ctas = (sms > 0 ? sms : 1) * (per_sm > 0 ? per_sm : 1);
         resident[dev].store(ctas, std::memory_order_relaxed);
     }
-    const uint32_t total = bw * bh;
-    constexpr uint32_t unit = L.tile_blocks;
-    const uint32_t units = (total + unit - 1) / unit;
-    const uint32_t grid = units < (uint32_t)ctas ? units : (uint32_t)ctas;
-    return launch_pdl(encode_image_tma<CODEC, BPT, COMPUTE, WORD>, dim3(grid), dim3(block), smem, stream, src, stride, dst,
-                      dst2, bw, 0xffffffffu / bw, total);
+    *out = ctas;
+    return cudaSuccess;
+}
+
+template <int CODEC, int BPT, int COMPUTE, bool WORD>
+cudaError_t launch_tma_t(const uint8_t* src, size_t stride, uint8_t* dst, uint8_t* dst2, uint32_t bw, uint32_t bh,
+                         cudaStream_t stream)
+{
+    constexpr TmaLayout L = tma_layout(COMPUTE, BPT, WORD);
+    const size_t smem = tma_smem_bytes(L);
+    const auto kernel = encode_image_tma<CODEC, BPT, COMPUTE, WORD>;
+    static std::atomic<int> resident[64];
+    int ctas = 0;
+    const cudaError_t e = resident_ctas_of(kernel, COMPUTE + 32, smem, resident, &ctas);
+    if (e != cudaSuccess) return e;
+    const uint32_t total = bw * bh, units = (total + L.tile_blocks - 1) / L.tile_blocks;
+    const uint32_t grid = std::min(units, (uint32_t)ctas);
+    return launch_pdl(kernel, dim3(grid), dim3(COMPUTE + 32), smem, stream, src, stride, dst, dst2, bw,
+                      0xffffffffu / bw, total);
 }
 
 template <int CODEC, int BPT>
@@ -624,6 +755,50 @@ cudaError_t launch_image_tma(int codec, const uint8_t* src, size_t stride, uint8
         if (tile.bpt == 2) return launch_tma_bpt<kBoth, 2>(src, stride, dst, dst2, bw, bh, tile.threads, stream);
     }
     return cudaErrorInvalidValue;
+}
+
+namespace {
+
+template <int CODEC, int BPT, int COMPUTE, bool WORD>
+cudaError_t launch_error_t(const uint8_t* blocks, const uint8_t* src, size_t stride, uint32_t bw, uint32_t bh,
+                           unsigned long long* sums, ErrorResult result, cudaStream_t stream)
+{
+    constexpr TmaLayout L = tma_layout(COMPUTE, BPT, WORD);
+    constexpr size_t smem = (size_t)L.stages * (L.stage_bytes + 16u) + (CODEC == kBC1 ? 0u : 32u * COMPUTE);
+    const auto kernel = error_image_tma<CODEC, BPT, COMPUTE, WORD>;
+    static std::atomic<int> resident[64];
+    int ctas = 0;
+    const cudaError_t e = resident_ctas_of(kernel, COMPUTE + 32, smem, resident, &ctas);
+    if (e != cudaSuccess) return e;
+    const uint32_t total = bw * bh, units = (total + L.tile_blocks - 1) / L.tile_blocks;
+    // a thread's sums hold kErrorSumBlocks blocks
+    const uint32_t least = (uint32_t)(((uint64_t)units * BPT + kErrorSumBlocks - 1) / kErrorSumBlocks);
+    const uint32_t grid = std::max(least, std::min(units, (uint32_t)ctas));
+    return launch_pdl(kernel, dim3(grid), dim3(COMPUTE + 32), smem, stream, blocks, src, stride, bw, 0xffffffffu / bw,
+                      total, sums, result);
+}
+
+template <int CODEC, bool WORD>
+cudaError_t launch_error(const uint8_t* blocks, const uint8_t* src, size_t stride, uint32_t bw, uint32_t bh,
+                         unsigned long long* sums, ErrorResult result, bool big, cudaStream_t stream)
+{
+    return big ? launch_error_t<CODEC, 2, 512, WORD>(blocks, src, stride, bw, bh, sums, result, stream)
+               : launch_error_t<CODEC, 1, 128, WORD>(blocks, src, stride, bw, bh, sums, result, stream);
+}
+
+}  // namespace
+
+cudaError_t launch_error_tma(int codec, const uint8_t* blocks, const uint8_t* src, uint32_t width, uint32_t height,
+                             size_t stride, bool vec16, bool big, unsigned long long* sums, ErrorResult result,
+                             cudaStream_t stream)
+{
+    const uint32_t bw = width / 4, bh = height / 4;
+    if (!vec16 && !word_rows_fit(big ? 1024 : 128, bw)) return cudaErrorInvalidValue;
+    if (codec == kBC1)
+        return vec16 ? launch_error<kBC1, false>(blocks, src, stride, bw, bh, sums, result, big, stream)
+                     : launch_error<kBC1, true>(blocks, src, stride, bw, bh, sums, result, big, stream);
+    return vec16 ? launch_error<kETC1S, false>(blocks, src, stride, bw, bh, sums, result, big, stream)
+                 : launch_error<kETC1S, true>(blocks, src, stride, bw, bh, sums, result, big, stream);
 }
 
 namespace {
