@@ -36,10 +36,14 @@ __device__ __forceinline__ void reduce_errors(const uint64_t (&in)[6], unsigned 
     sync();
     if (threadIdx.x == 0) last = atomicAdd(result.finished, 1u) == gridDim.x - 1u;
     sync();
-    if (!last) return;
+    if (!last || warp != 0) return;
     __threadfence();  // every CTA's sums after the last tick
-    if (threadIdx.x < 6) result.host[threadIdx.x] = atomicExch(&sums[threadIdx.x], 0ull);
-    if (threadIdx.x == 0) *result.finished = 0u;
+    if (lane < 6) result.host[lane] = atomicExch(&sums[lane], 0ull);
+    if (lane == 6) *result.finished = 0u;
+    __threadfence_system();  // before the word that the host polls
+    __syncwarp();
+    if (lane == 0)
+        asm volatile("st.release.sys.global.u32 [%0], %1;" ::"l"(result.flag), "r"(result.serial) : "memory");
 }
 
 }  // namespace goofy_gpu
