@@ -16,6 +16,7 @@ over the C ABI of ``libgoofy_gb300.so`` (include/goofy_gpu.h):
 """
 import ctypes
 import os
+import struct
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(HERE, "_build", "libgoofy_gb300.so")
@@ -227,6 +228,9 @@ def synth_lib():
     return _synth
 
 
+_CHAR_AT = ctypes.c_char.from_buffer
+
+
 def _addr(buf):
     """Address of a host buffer: numpy array, bytearray, ctypes object or int."""
     if buf is None:
@@ -234,7 +238,10 @@ def _addr(buf):
     if isinstance(buf, int):
         return buf
     if hasattr(buf, "ctypes"):  # numpy
-        return buf.ctypes.data
+        try:  # 0.25 us where buf.ctypes.data takes 1.5; needs a writable, C-contiguous array that is not empty
+            return ctypes.addressof(_CHAR_AT(buf))
+        except (TypeError, ValueError, BufferError):
+            return buf.__array_interface__["data"][0]
     if isinstance(buf, bytearray):
         return ctypes.addressof((ctypes.c_char * len(buf)).from_buffer(buf))
     if hasattr(buf, "data_ptr"):  # torch tensor
@@ -608,6 +615,11 @@ def psnr_rgb(codec, blocks, src, width, height, stride):
     return rc, out.value, sums
 
 
+_QUALITY_NAMES = [n for n, _ in Quality._fields_]
+_QUALITY_VALUES = struct.Struct("=14dQ")
+assert _QUALITY_VALUES.size == ctypes.sizeof(Quality)
+
+
 def mse_psnr(codec, blocks, src, width, height, stride):
     """The harness's getMsePsnr of device `src` against its decoded device
     `blocks`, computed on the GPU; a dict of the MsePsnr fields."""
@@ -615,7 +627,7 @@ def mse_psnr(codec, blocks, src, width, height, stride):
     rc = lib().goofy_gpu_mse_psnr(codec, _addr(blocks), _addr(src), width, height, stride, ctypes.byref(q))
     if rc != OK:
         raise RuntimeError("mse_psnr: %s %s" % (status_string(rc), last_error()))
-    return {n: getattr(q, n) for n, _ in Quality._fields_}
+    return dict(zip(_QUALITY_NAMES, _QUALITY_VALUES.unpack_from(q)))
 
 
 def container(codec, levels):
@@ -637,16 +649,20 @@ def container(codec, levels):
     return out.tobytes()
 
 
+_LEVELS = Level * 32  # more than any chain has
+_LEVEL_VALUES = struct.Struct("=QIII4x")
+assert _LEVEL_VALUES.size == ctypes.sizeof(Level)
+
+
 def generate_mips(src, width, height, stride, arena, arena_bytes, stream=None):
     """Device mip chain of `src` into `arena`; returns [(ptr, w, h, stride), ...] (level 0 = src)."""
-    n = lib().goofy_gpu_mip_count(width, height)
-    levels = (Level * max(n, 1))()
+    levels = _LEVELS()
     count = ctypes.c_uint32()
     rc = lib().goofy_gpu_generate_mips(_addr(src), width, height, stride, _addr(arena), arena_bytes, levels,
-                                       max(n, 1), ctypes.byref(count), stream)
+                                       len(levels), ctypes.byref(count), stream)
     if rc != OK:
         raise RuntimeError("generate_mips: %s %s" % (status_string(rc), last_error()))
-    return [(levels[i].data, levels[i].width, levels[i].height, levels[i].stride) for i in range(count.value)]
+    return list(_LEVEL_VALUES.iter_unpack(ctypes.string_at(levels, _LEVEL_VALUES.size * count.value)))
 
 
 def read_png(source, opaque=True, stride=None):
