@@ -31,28 +31,42 @@ namespace goofy_gpu {
 // constant so that a pixel's palette address is a shift and an add.
 constexpr uint32_t kDecodeThreads = 256;
 
-template <int CODEC>
+// N blocks a thread, 32 apart, so each store of a warp writes 512 contiguous
+// bytes of a pixel row.
+template <int CODEC, int N>
 __global__ void __launch_bounds__(kDecodeThreads) decode_image_kernel(const uint8_t* __restrict__ blocks, uint32_t bw,
-                                                           uint32_t nblk, uint8_t* __restrict__ rgba, size_t stride,
-                                                           unsigned long long* __restrict__ unsupported)
+                                                                      uint32_t bw_magic, uint32_t nblk,
+                                                                      uint8_t* __restrict__ rgba, size_t stride,
+                                                                      unsigned long long* __restrict__ unsupported)
 {
     pdl_launch_dependents();
-    __shared__ uint32_t pal[8 * kDecodeThreads];
-    const uint32_t i = blockIdx.x * kDecodeThreads + threadIdx.x;
-    bool ok = true;
+    __shared__ uint32_t pal[CODEC == kBC1 ? 1 : 8 * kDecodeThreads];
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t i0 = (blockIdx.x * (kDecodeThreads / 32u) + (threadIdx.x >> 5)) * (32u * N) + lane;
+    uint2 code[N];
+    uint32_t bad = 0;
     pdl_wait();
-    if (i < nblk) {
-        const uint32_t by = i / bw, bx = i - by * bw;
-        uint32_t px[16];
-        ok = decode_block<CODEC>(load_block8(blocks + 8u * (size_t)i), pal + threadIdx.x, kDecodeThreads, px);
-        uint8_t* row = rgba + (size_t)by * 4u * stride + 16u * (size_t)bx;
 #pragma unroll
-        for (int y = 0; y < 4; ++y)
-            *reinterpret_cast<uint4*>(row + (size_t)y * stride) = make_uint4(px[4 * y], px[4 * y + 1], px[4 * y + 2],
-                                                                             px[4 * y + 3]);
+    for (int j = 0; j < N; ++j)
+        code[j] = i0 + 32u * j < nblk ? load_block8(blocks + 8u * (size_t)(i0 + 32u * j)) : make_uint2(0u, 0u);
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+        const uint32_t i = i0 + 32u * j;
+        if (i < nblk) {
+            uint32_t bx, px[16];
+            const uint32_t by = div_magic(i, bw, bw_magic, bx);
+            if (!decode_block<CODEC>(code[j], pal + threadIdx.x, kDecodeThreads, px)) ++bad;
+            uint8_t* row = rgba + (size_t)by * 4u * stride + 16u * (size_t)bx;
+#pragma unroll
+            for (int y = 0; y < 4; ++y)
+                *reinterpret_cast<uint4*>(row + (size_t)y * stride) = make_uint4(px[4 * y], px[4 * y + 1], px[4 * y + 2],
+                                                                                 px[4 * y + 3]);
+        }
     }
-    const unsigned bad = __ballot_sync(0xffffffffu, !ok);
-    if (bad && (threadIdx.x & 31u) == 0) atomicAdd(unsupported, (unsigned long long)__popc(bad));
+    if constexpr (CODEC != kBC1) {
+        bad = __reduce_add_sync(0xffffffffu, bad);
+        if (bad && lane == 0) atomicAdd(unsupported, (unsigned long long)bad);
+    }
 }
 
 // Tiny images and narrow rows; the others take error_image_tma (encode_tma.cu).
@@ -163,17 +177,34 @@ cudaError_t launch_quality_batch(const BatchImage* images, uint32_t n_images, co
     return cudaGetLastError();
 }
 
+namespace {
+
+template <int CODEC, int N>
+cudaError_t launch_decode_t(const uint8_t* blocks, uint32_t bw, uint32_t nblk, uint8_t* rgba, size_t stride,
+                            unsigned long long* unsupported, cudaStream_t stream)
+{
+    const uint32_t grid = (nblk + N * kDecodeThreads - 1) / (N * kDecodeThreads);
+    return launch_pdl(decode_image_kernel<CODEC, N>, dim3(grid), dim3(kDecodeThreads), 0, stream, blocks, bw,
+                      0xffffffffu / bw, nblk, rgba, stride, unsupported);
+}
+
+}  // namespace
+
 cudaError_t launch_decode(int codec, const uint8_t* blocks, uint32_t width, uint32_t height, uint8_t* rgba,
                           size_t stride, unsigned long long* unsupported, cudaStream_t stream)
 {
     const uint32_t bw = width / 4, nblk = bw * (height / 4);
     if (nblk == 0) return cudaSuccess;
-    const uint32_t grid = (nblk + kDecodeThreads - 1) / kDecodeThreads;
+    // A wave is 152 SMs x 2048 threads = 311296 blocks.  Two blocks a thread where one would leave a second wave
+    // mostly empty, up to two full waves of two (us, one / two, BC1 and ETC1s): 3840x2160 (518400 blocks) 6.3 / 6.1
+    // and 6.5 / 6.2, 4096^2 (1048576) 12.0 / 11.6 and 12.2 / 11.7.  Below and above one is as fast or faster: 3000x2048
+    // (384000) 4.8 / 5.4 and 5.0 / 5.6, 5000x4096 (1280000) 14.7 / 14.6 and 14.8 / 14.7, 8192^2 44.2 / 44.7 and 44.8 / 44.9.
+    const bool two = nblk >= 430000 && nblk <= 1250000;
     if (codec == kBC1)
-        return launch_pdl(decode_image_kernel<kBC1>, dim3(grid), dim3(kDecodeThreads), 0, stream, blocks, bw, nblk, rgba, stride,
-                          unsupported);
-    return launch_pdl(decode_image_kernel<kETC1S>, dim3(grid), dim3(kDecodeThreads), 0, stream, blocks, bw, nblk, rgba, stride,
-                      unsupported);
+        return two ? launch_decode_t<kBC1, 2>(blocks, bw, nblk, rgba, stride, unsupported, stream)
+                   : launch_decode_t<kBC1, 1>(blocks, bw, nblk, rgba, stride, unsupported, stream);
+    return two ? launch_decode_t<kETC1S, 2>(blocks, bw, nblk, rgba, stride, unsupported, stream)
+               : launch_decode_t<kETC1S, 1>(blocks, bw, nblk, rgba, stride, unsupported, stream);
 }
 
 namespace {

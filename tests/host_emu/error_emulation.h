@@ -1,4 +1,4 @@
-// error_emulation.h -- TEST ONLY.  CPU definitions of the further intrinsics
+// error_emulation.h -- TEST ONLY.  CPU definition of the further intrinsic
 // block_error.cuh uses.
 #pragma once
 #include <cstdint>
@@ -13,12 +13,3 @@ static inline uint32_t __vabsdiffu4(uint32_t a, uint32_t b)
     }
     return r;
 }
-
-namespace goofy_gpu {
-// prmt.b32 with selector nibbles 0..7; fails on any other
-static inline uint32_t pick(uint32_t a, uint32_t b, uint32_t sel)
-{
-    if (sel & 0x8888u) __builtin_trap();
-    return __byte_perm(a, b, sel);
-}
-}  // namespace goofy_gpu
