@@ -217,10 +217,13 @@ void retire_locked(goofy_gpu_server* s)
             cudaEventElapsedTime(&span_ms, sl.ev_first, sl.ev_last) != cudaSuccess)
             cudaGetLastError();
         const uint64_t kernel_ns = (uint64_t)(k_ms * 1e6f), total_ns = (uint64_t)(sl.t_callback - sl.t_enqueue);
+        // the callback can run before the enqueueing thread has read its clock: count no more than the launch took
+        const uint64_t enqueue_ns = std::min(sl.enqueue_ns, total_ns > 0 ? total_ns - 1 : 0);
         s->max_kernel_ns = std::max(s->max_kernel_ns, kernel_ns);
+        s->max_enqueue_ns = std::max(s->max_enqueue_ns, enqueue_ns);
         if (total_ns > s->max_launch_ns) {
             s->max_launch_ns = total_ns;
-            s->slowest_enqueue_ns = sl.enqueue_ns;
+            s->slowest_enqueue_ns = enqueue_ns;
             s->slowest_gpu_span_ns = (uint64_t)(span_ms * 1e6f);
             s->slowest_kernel_ns = kernel_ns;
         }
@@ -356,7 +359,6 @@ int launch(goofy_gpu_server* s, int si, const std::vector<uint64_t>& tickets, Ca
     {
         std::lock_guard<std::mutex> lk(s->mu);
         sl.enqueue_ns = enq;  // the scheduler retires this launch only after launch() returns
-        s->max_enqueue_ns = std::max(s->max_enqueue_ns, enq);
         if (poll) s->polling.push_back(cb->slot);
     }
     if (poll) s->cv_poll.notify_one();
