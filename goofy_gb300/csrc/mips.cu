@@ -8,8 +8,9 @@
 // being copied instead of halved -- the rule of the workload generator's
 // goofy_synth_downsample, so device and host chains are bit-identical.  While
 // both axes halve, one launch makes up to 6 levels from shared-memory tiles
-// (mip_fused_kernel); the rest take one launch per level, a thread per output
-// pixel.  Channel pairs are summed in 16-bit lanes.
+// (mip_fused_kernel); small levels behind them take one launch in all
+// (mip_tail_kernel), larger ones a launch each, a thread per output pixel.
+// Channel pairs are summed in 16-bit lanes.
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -152,6 +153,57 @@ __global__ void __launch_bounds__(256) mip_fused_kernel(const uint8_t* __restric
     for (int k = 0; k < TILES; ++k) mip_tile(r[k], act, blockIdx.x * TILES + k, ty, tw_log2, th_log2, nlev, out, buf);
 }
 
+// The end of a chain in one CTA: levels of at most kTailPixels pixels, each
+// made from the one above, which is kept in shared memory.  Used where the
+// fused kernel would not reach the chain's last level, because one axis is at
+// 4 first and the rest would take a launch a level.  Whole chains (us), a
+// launch a level / one: 4096x256 5.7 / 4.3, 1024x256 3.4 / 3.0, 4096x1024 7.1 /
+// 6.2, 64x16 2.7 / 1.7, 8192x64 9.9 / 6.9, and 1.5 us of host time a launch.
+constexpr uint32_t kTailPixels = 4096, kTailLevels = 16, kTailThreads = 512;
+struct TailOut {
+    uint8_t* data[kTailLevels];
+    uint32_t pitch[kTailLevels];
+};
+
+__global__ void __launch_bounds__(kTailThreads) mip_tail_kernel(const uint8_t* __restrict__ src, size_t src_stride,
+                                                                uint32_t w, uint32_t h, uint32_t nlev,
+                                                                const __grid_constant__ TailOut out)
+{
+    goofy_gpu::pdl_launch_dependents();
+    __shared__ uint32_t buf[2][kTailPixels];
+    goofy_gpu::pdl_wait();
+    for (uint32_t l = 0; l < nlev; ++l) {
+        const uint32_t fx = w > 4 ? 2 : 1, fy = h > 4 ? 2 : 1, dw = w / fx, dh = h / fy;
+        const uint32_t* in = buf[(l + 1) & 1];
+        uint32_t* next = buf[l & 1];
+        for (uint32_t t = threadIdx.x; t < dw * dh; t += kTailThreads) {
+            const uint32_t x = t & (dw - 1u), y = t / dw;
+            uint32_t a, b, c, d;
+            if (l == 0) {
+                const uint8_t* r0 = src + (size_t)(y * fy) * src_stride + 4u * (size_t)(x * fx);
+                const uint8_t* r1 = r0 + src_stride * (fy - 1);
+                a = __ldg(reinterpret_cast<const uint32_t*>(r0));
+                b = __ldg(reinterpret_cast<const uint32_t*>(r0 + 4 * (fx - 1)));
+                c = __ldg(reinterpret_cast<const uint32_t*>(r1));
+                d = __ldg(reinterpret_cast<const uint32_t*>(r1 + 4 * (fx - 1)));
+            } else {
+                const uint32_t* r0 = in + (y * fy) * w + x * fx;
+                const uint32_t* r1 = r0 + w * (fy - 1);
+                a = r0[0];
+                b = r0[fx - 1];
+                c = r1[0];
+                d = r1[fx - 1];
+            }
+            const uint32_t v = box4(a, b, c, d);
+            next[t] = v;
+            *reinterpret_cast<uint32_t*>(out.data[l] + (size_t)y * out.pitch[l] + 4u * x) = v;
+        }
+        w = dw;
+        h = dh;
+        __syncthreads();
+    }
+}
+
 bool pow2(uint32_t v) { return v && !(v & (v - 1)); }
 
 uint32_t log2u(uint32_t v)
@@ -227,6 +279,18 @@ GOOFY_EXPORT int goofy_gpu_generate_mips(const void* src, uint32_t width, uint32
         // square tiles of 2^f pixels make exactly f levels (one pixel of the last);
         // the tail of a chain thus gets many small tiles instead of a few large ones
         const uint32_t tw = 1u << f, th = 1u << f;
+        const goofy_gpu_level& lv = levels[i];
+        if (n - i > 1 && f < n - i && n - i <= kTailLevels && (uint64_t)lv.width * lv.height <= kTailPixels) {
+            TailOut to{};
+            for (uint32_t l = 0; i + l < n; ++l) {
+                to.data[l] = static_cast<uint8_t*>(levels[i + l].data);
+                to.pitch[l] = levels[i + l].stride;
+            }
+            GOOFY_CUDA_TRY(goofy_gpu::launch_pdl(mip_tail_kernel, dim3(1), dim3(kTailThreads), 0, st,
+                                                 static_cast<const uint8_t*>(up.data), (size_t)up.stride, up.width,
+                                                 up.height, n - i, to));
+            break;
+        }
         if (f >= 2 && reinterpret_cast<uintptr_t>(up.data) % 16 == 0 && up.stride % 16 == 0) {
             MipOut mo{};
             for (uint32_t l = 0; l < f; ++l) {
@@ -245,7 +309,6 @@ GOOFY_EXPORT int goofy_gpu_generate_mips(const void* src, uint32_t width, uint32
             i += f;
             continue;
         }
-        const goofy_gpu_level& lv = levels[i];
         const uint32_t fx = up.width > lv.width ? 2 : 1, fy = up.height > lv.height ? 2 : 1;
         const bool pair = fx == 2 && reinterpret_cast<uintptr_t>(up.data) % 8 == 0 && up.stride % 8 == 0;
         const dim3 grid((lv.width + 255) / 256, lv.height);
