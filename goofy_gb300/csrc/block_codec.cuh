@@ -337,24 +337,48 @@ GOOFY_FN uint2 encode_etc1s(const uint32_t (&w)[16], const uint8_t* ctrl_lut)
     return etc1s_from_extents(w, l, lane_extents(l), ctrl_lut);
 }
 
+// The index word of a block from that of the block with its columns x in the
+// places x ^ q (q in 0..3).  Everything else of a block is the same for both:
+// the extents are symmetric in all pixels, and the ETC1s mean tree pairs the
+// columns as {{0, 1}, {2, 3}}, which x ^ q maps onto itself, by averages that
+// are symmetric in their two sides.  BC1: 2-bit fields and nibbles of a byte
+// trade places; ETC1s (bits 4(x ^ 2) + y of each half): nibbles and bytes.
+template <int CODEC>
+GOOFY_FN uint32_t swap_columns(uint32_t idx, uint32_t q)
+{
+    if constexpr (CODEC == kBC1) {
+        if (q & 1u) idx = ((idx >> 2) & 0x33333333u) | ((idx & 0x33333333u) << 2);
+        return (q & 2u) ? ((idx >> 4) & 0x0f0f0f0fu) | ((idx & 0x0f0f0f0fu) << 4) : idx;
+    } else {
+        if (q & 1u) idx = ((idx >> 4) & 0x0f0f0f0fu) | ((idx & 0x0f0f0f0fu) << 4);
+        return perm(idx, 0u, (q & 2u) ? 0x2301u : 0x3210u);
+    }
+}
+
 // Both codecs from one set of lanes and extents: the R/B masks, the min / max
 // trees and the brightness statistics are computed once, and the ETC1s index
 // word is a bit permutation of the BC1 one.  {BC1 block, ETC1s block}, each
-// bit-identical to its own encoder's.
-GOOFY_FN uint4 encode_both(const uint32_t (&w)[16], const uint8_t* ctrl_lut)
+// bit-identical to its own encoder's.  XORED: w holds the columns at x ^ q.
+template <bool XORED = false>
+GOOFY_FN uint4 encode_both(const uint32_t (&w)[16], const uint8_t* ctrl_lut, uint32_t q = 0u)
 {
     BlockLanes l;
     block_lanes(w, l);
     const Extents e = lane_extents(l);
-    const uint2 a = bc1_from_extents(w, e), b = etc1s_from_extents<true>(w, l, e, ctrl_lut);
+    uint2 a = bc1_from_extents(w, e);
+    const uint2 b = etc1s_from_extents<true>(w, l, e, ctrl_lut);
+    if constexpr (XORED) a.y = swap_columns<kBC1>(a.y, q);
     return make_uint4(a.x, a.y, b.x, etc1s_indices_from_bc1(a.y));
 }
 
-template <int CODEC>
-GOOFY_FN uint2 encode_block(const uint32_t (&w)[16], const uint8_t* ctrl_lut)
+template <int CODEC, bool XORED = false>
+GOOFY_FN uint2 encode_block(const uint32_t (&w)[16], const uint8_t* ctrl_lut, uint32_t q = 0u)
 {
-    if constexpr (CODEC == kBC1) return encode_bc1(w);
-    else return encode_etc1s(w, ctrl_lut);
+    uint2 e;
+    if constexpr (CODEC == kBC1) e = encode_bc1(w);
+    else e = encode_etc1s(w, ctrl_lut);
+    if constexpr (XORED) e.y = swap_columns<CODEC>(e.y, q);
+    return e;
 }
 
 }  // namespace goofy_gpu

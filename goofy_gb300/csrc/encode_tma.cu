@@ -34,10 +34,12 @@
 // shift is taken out when the words leave shared memory.  The
 // register-loading kernel reads such a block with sixteen 4-byte loads that
 // skip L1, so every 32-byte sector crosses L2 up to four times: 1996x1532
-// ETC1s 7.3-11.0 us there, 5.2 us here; 4096^2 (over 400 MB of inputs) BC1 15.8,
-// ETC1s 17.0 there with the best CTA size, 13.1 and 14.1 here.  Every wait is bounded (async_copy.cuh): a stuck
-// barrier ends the kernel with a counted time-out instead of a hang, and the
-// producer then waits (bounded) for the copies it issued before its CTA exits.
+// ETC1s 7.3-11.0 us there, 4.6 us here; 4096^2 (over 400 MB of inputs) BC1 15.8,
+// ETC1s 17.0 there with the best CTA size, 12.2 and 13.9 here.
+//
+// Every wait is bounded (async_copy.cuh): a stuck barrier ends the kernel with
+// a counted time-out instead of a hang, and the producer then waits (bounded)
+// for the copies it issued before its CTA exits.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -120,11 +122,17 @@ __host__ __device__ constexpr uint32_t l2_prefetch_tiles(const TmaLayout& l)
 // writes while the stage is held, and its result is dropped.  Only the
 // stores are conditional, so the loads and the codec run without branches.
 // WORD: block k's pixel row y starts shift[y] bytes into granule
-// k + (its block row - the unit's first) of plane y and is read word by word
-// (four lanes a bank, 64 wavefronts a warp and block instead of 16, which the
-// load/store unit has room for; picking the words out of two 16-byte loads
-// would take 36 selects a block on the busy ALU pipe).
-template <int BPT, bool WORD>
+// k + (its block row - the unit's first) of plane y and is read word by word.
+// In column order that puts four lanes on a bank (64 wavefronts a warp and
+// block instead of 16), so with XOR_COLUMNS lane l reads column x ^ (l >> 3)
+// into w[4y + x]: the eight lanes of a group are 4 words apart and the four
+// groups a word apart, so no two share a bank.  The codec gives the same block
+// but for the order of its indices (swap_columns in block_codec.cuh).
+// Measured against column order (400 MB of inputs): 4096^2 BC1 13.2 -> 12.2,
+// ETC1s 14.1 -> 13.9 us; 1996x1532 4.4 -> 4.1 and 5.0 -> 4.6.  Four addresses
+// a block plus uniform row offsets: added the other way round (a row's base
+// plus the column) the sixteen sums cost more than the conflicts at 2376x2628.
+template <int BPT, bool WORD, bool XOR_COLUMNS>
 __device__ __forceinline__ void load_stage(const uint8_t* buf, uint32_t row_bytes, uint32_t warp, uint32_t lane,
                                            uint32_t nb, uint32_t bx0, uint32_t bw, uint32_t bw_magic,
                                            const uint32_t (&shift)[4], uint32_t (&w)[BPT][16])
@@ -136,11 +144,13 @@ __device__ __forceinline__ void load_stage(const uint8_t* buf, uint32_t row_byte
             uint32_t x;
             const uint32_t s = div_magic(min(bx0 + b, bx0 + nb - 1u), bw, bw_magic, x);
             const uint8_t* p = buf + 16u * (min(b, nb - 1u) + s);
+            const uint32_t q = XOR_COLUMNS ? (lane >> 1) & 12u : 0u;
+            const uint8_t* const col[4] = {p + q, p + (q ^ 4u), p + (q ^ 8u), p + (q ^ 12u)};
 #pragma unroll
             for (int r = 0; r < 4; ++r)
 #pragma unroll
                 for (int i = 0; i < 4; ++i)
-                    w[j][4 * r + i] = *reinterpret_cast<const uint32_t*>(p + r * row_bytes + shift[r] + 4 * i);
+                    w[j][4 * r + i] = *reinterpret_cast<const uint32_t*>(col[i] + (r * row_bytes + shift[r]));
         } else {
 #pragma unroll
             for (int r = 0; r < 4; ++r) {
@@ -161,18 +171,19 @@ __device__ __forceinline__ void encode_stage(const uint8_t* buf, uint32_t row_by
                                              const uint32_t (&shift)[4])
 {
     uint32_t w[BPT][16];
-    load_stage<BPT, WORD>(buf, row_bytes, warp, lane, nb, bx0, bw, bw_magic, shift, w);
+    load_stage<BPT, WORD, WORD>(buf, row_bytes, warp, lane, nb, bx0, bw, bw_magic, shift, w);
+    const uint32_t q = WORD ? lane >> 3 : 0u;
 #pragma unroll
     for (int j = 0; j < BPT; ++j) {
         const uint32_t b = (warp * BPT + j) * 32u + lane;
         if constexpr (CODEC == kBoth) {
-            const uint4 e = encode_both(w[j], ctrl_lut);
+            const uint4 e = encode_both<WORD>(w[j], ctrl_lut, q);
             if (b < nb) {
                 st_stream8(out + 8u * (size_t)b, make_uint2(e.x, e.y));
                 st_stream8(out2 + 8u * (size_t)b, make_uint2(e.z, e.w));
             }
         } else {
-            const uint2 e = encode_block<CODEC>(w[j], ctrl_lut);
+            const uint2 e = encode_block<CODEC, WORD>(w[j], ctrl_lut, q);
             if (b < nb) st_stream8(out + 8u * (size_t)b, e);
         }
     }
@@ -424,7 +435,7 @@ __global__ void __launch_bounds__(COMPUTE + 32, BPT == 2 ? 1 : CODEC == kBC1 ? 6
         const uint32_t nb = min(unit, total - first);
         uint32_t bx0 = 0, w[BPT][16];
         if constexpr (WORD) div_magic(first, bw, bw_magic, bx0);
-        load_stage<BPT, WORD>(smem + slot * L.stage_bytes, L.row_bytes, warp, lane, nb, bx0, bw, bw_magic, im.shift, w);
+        load_stage<BPT, WORD, false>(smem + slot * L.stage_bytes, L.row_bytes, warp, lane, nb, bx0, bw, bw_magic, im.shift, w);
 #pragma unroll
         for (int j = 0; j < BPT; ++j)
             if ((warp * BPT + j) * 32u + lane < nb)
