@@ -8,7 +8,8 @@
 // being copied instead of halved -- the rule of the workload generator's
 // goofy_synth_downsample, so device and host chains are bit-identical.  While
 // both axes halve, one launch makes up to 6 levels from shared-memory tiles
-// (mip_fused_kernel); small levels behind them take one launch in all
+// (mip_fused_kernel), or the whole chain of 512^2 and 1024^2
+// (mip_chain_kernel); small levels behind them take one launch in all
 // (mip_tail_kernel), larger ones a launch each, a thread per output pixel.
 // Channel pairs are summed in 16-bit lanes.
 #include <cuda_runtime.h>
@@ -67,21 +68,27 @@ __global__ void __launch_bounds__(256) mip_level_kernel(const uint8_t* __restric
 // the remaining levels (at most 8x8 pixels per tile) go through shared
 // memory.  Used while both axes halve; every level is the same box4 of the
 // level above as in the one-level kernel, so the results are identical.
-struct MipOut {
-    uint8_t* data[6];
-    uint32_t pitch[6];
+template <int LEVELS>
+struct MipLevels {
+    uint8_t* data[LEVELS];
+    uint32_t pitch[LEVELS];
 };
+using MipOut = MipLevels<6>;
 
-__device__ __forceinline__ void store_px(const MipOut& o, int l, uint32_t row, uint32_t col, uint32_t v)
+template <typename Out>
+__device__ __forceinline__ void store_px(const Out& o, int l, uint32_t row, uint32_t col, uint32_t v)
 {
     *reinterpret_cast<uint32_t*>(o.data[l] + (size_t)row * o.pitch[l] + 4u * col) = v;
 }
 
-// One tile's levels from its thread's 4x4 patch `r` (already loaded).
-__device__ __forceinline__ void mip_tile(const uint4 (&r)[4], bool act, uint32_t tx, uint32_t ty, uint32_t tw_log2,
-                                         uint32_t th_log2, uint32_t nlev, const MipOut& out, uint32_t (*buf)[64])
+// One tile's levels from the 4x4 patches `r` (already loaded) of its 256
+// threads, of which this is number t.  Returns thread 0's pixel of the sixth
+// level, if there is one.  A CTA calls it for all its tiles at once.
+template <typename Out>
+__device__ __forceinline__ uint32_t mip_tile(const uint4 (&r)[4], uint32_t t, bool act, uint32_t tx, uint32_t ty,
+                                             uint32_t tw_log2, uint32_t th_log2, uint32_t nlev, const Out& out,
+                                             uint32_t (*buf)[64])
 {
-    const uint32_t t = threadIdx.x;
     const uint32_t w2_log2 = tw_log2 - 2, h2_log2 = th_log2 - 2, w2 = 1u << w2_log2;
     const uint32_t x2 = t & (w2 - 1u), y2 = t >> w2_log2;
     uint32_t v2 = 0;
@@ -94,7 +101,7 @@ __device__ __forceinline__ void mip_tile(const uint4 (&r)[4], bool act, uint32_t
         v2 = box4(q00, q01, q10, q11);
         if (nlev > 1) store_px(out, 1, (ty << h2_log2) + y2, (tx << w2_log2) + x2, v2);
     }
-    if (nlev <= 2) return;
+    if (nlev <= 2) return 0;
     // third level: lanes with even x2 and y2 combine their 2x2 neighbourhood
     const uint32_t b = __shfl_xor_sync(0xffffffffu, v2, 1), c = __shfl_xor_sync(0xffffffffu, v2, w2),
                    d = __shfl_xor_sync(0xffffffffu, v2, w2 ^ 1u);
@@ -104,7 +111,7 @@ __device__ __forceinline__ void mip_tile(const uint4 (&r)[4], bool act, uint32_t
         store_px(out, 2, (ty << h3_log2) + y3, (tx << w3_log2) + x3, v3);
         buf[0][(y3 << w3_log2) + x3] = v3;
     }
-    uint32_t cw_log2 = w3_log2, ch_log2 = h3_log2;
+    uint32_t cw_log2 = w3_log2, ch_log2 = h3_log2, v = 0;
 #pragma unroll
     for (uint32_t l = 3; l < 6; ++l) {  // unrolled: the level indexes `out` as a constant (no stack copy)
         if (l >= nlev) break;
@@ -115,7 +122,7 @@ __device__ __forceinline__ void mip_tile(const uint4 (&r)[4], bool act, uint32_t
         if (t < (1u << (nw_log2 + nh_log2))) {
             const uint32_t ox = t & ((1u << nw_log2) - 1u), oy = t >> nw_log2;
             const uint32_t* r0 = in + (2u * oy) * cw + 2u * ox;
-            const uint32_t v = box4(r0[0], r0[1], r0[cw], r0[cw + 1]);
+            v = box4(r0[0], r0[1], r0[cw], r0[cw + 1]);
             next[t] = v;
             store_px(out, (int)l, (ty << nh_log2) + oy, (tx << nw_log2) + ox, v);
         }
@@ -123,6 +130,7 @@ __device__ __forceinline__ void mip_tile(const uint4 (&r)[4], bool act, uint32_t
         ch_log2 = nh_log2;
     }
     __syncthreads();  // the next tile of this CTA reuses buf
+    return v;
 }
 
 // TILES horizontally adjacent tiles per CTA: every patch load of all of them
@@ -150,7 +158,67 @@ __global__ void __launch_bounds__(256) mip_fused_kernel(const uint8_t* __restric
         }
     }
 #pragma unroll
-    for (int k = 0; k < TILES; ++k) mip_tile(r[k], act, blockIdx.x * TILES + k, ty, tw_log2, th_log2, nlev, out, buf);
+    for (int k = 0; k < TILES; ++k) mip_tile(r[k], t, act, blockIdx.x * TILES + k, ty, tw_log2, th_log2, nlev, out, buf);
+}
+
+// Whole square chains of 7 and 8 levels (512^2, 1024^2) in one launch: a
+// cluster of CTAs takes a square of K x K tiles of 64x64 pixels, 256 threads a
+// tile; each tile's last pixel goes to the first CTA's shared memory, and that
+// CTA makes the levels above.  Against two launches, mips / mips and the
+// encode behind them (us): 512^2 2.55 / 4.36 -> 2.12 / 3.71, 1024^2 3.52 / 6.88 ->
+// 3.14 / 5.16, and 1.5 us of host time.  2048^2 stays at two launches (5.7 us
+// for the mips): as 16 clusters of 64 tiles it took 6.5 (16 CTAs of 512
+// threads) to 10 us, clusters that large leaving SMs without one.
+__host__ __device__ constexpr int chain_cluster(int k) { return k == 2 ? 4 : 8; }
+__host__ __device__ constexpr int chain_tiles(int k) { return k * k / chain_cluster(k); }  // a CTA's
+__host__ __device__ constexpr int chain_levels(int k) { return k == 2 ? 7 : 8; }
+
+template <int K>
+__global__ void __cluster_dims__(chain_cluster(K), 1, 1) __launch_bounds__(256 * chain_tiles(K), 1)
+    mip_chain_kernel(const uint8_t* __restrict__ src, size_t src_stride, uint32_t squares_x,
+                     const __grid_constant__ MipLevels<chain_levels(K)> out)
+{
+    goofy_gpu::pdl_launch_dependents();
+    constexpr uint32_t kCtas = chain_cluster(K);
+    __shared__ uint32_t buf[chain_tiles(K)][2][64];
+    __shared__ uint32_t top[K * K];  // the first CTA's: the tiles' last pixels
+    const uint32_t group = threadIdx.x >> 8, t = threadIdx.x & 255u, rank = blockIdx.x % kCtas;
+    const uint32_t square = blockIdx.x / kCtas, sx = square % squares_x, sy = square / squares_x;
+    const uint32_t tile = rank * chain_tiles(K) + group, tx = sx * K + tile % K, ty = sy * K + tile / K;
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+    const uint8_t* patch = src + (size_t)(64u * ty + 4u * (t >> 4)) * src_stride + 4u * (64u * tx + 4u * (t & 15u));
+    goofy_gpu::pdl_wait();
+    uint4 r[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) r[j] = __ldg(reinterpret_cast<const uint4*>(patch + (size_t)j * src_stride));
+    const uint32_t last = mip_tile(r, t, true, tx, ty, 6u, 6u, 6u, out, buf[group]);
+    asm volatile("barrier.cluster.wait.aligned;" ::: "memory");  // the first CTA has started
+    if (t == 0) {
+        uint32_t at = (uint32_t)__cvta_generic_to_shared(&top[tile]), remote;
+        asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(remote) : "r"(at));
+        asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(remote), "r"(last) : "memory");
+    }
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    if (rank != 0) return;
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if (threadIdx.x >= 32) return;
+    constexpr uint32_t n = K / 2;
+    const uint32_t lane = threadIdx.x, x = lane % n, y = lane / n;
+    uint32_t v = 0;
+    if (lane < n * n) {
+        const uint32_t* p = top + 2u * y * K + 2u * x;
+        v = box4(p[0], p[1], p[K], p[K + 1]);
+        store_px(out, 6, sy * n + y, sx * n + x, v);
+    }
+#pragma unroll
+    for (uint32_t d = 1, l = 7; 2 * d <= n; d *= 2, ++l) {  // neighbours are d pixels apart
+        const uint32_t b = __shfl_xor_sync(0xffffffffu, v, d), c = __shfl_xor_sync(0xffffffffu, v, d * n),
+                       e = __shfl_xor_sync(0xffffffffu, v, d * n ^ d);
+        v = box4(v, b, c, e);
+        if (lane < n * n && !(x & (2 * d - 1)) && !(y & (2 * d - 1)))
+            store_px(out, (int)l, sy * (n / (2 * d)) + y / (2 * d), sx * (n / (2 * d)) + x / (2 * d), v);
+    }
 }
 
 // The end of a chain in one CTA: levels of at most kTailPixels pixels, each
@@ -202,6 +270,20 @@ __global__ void __launch_bounds__(kTailThreads) mip_tail_kernel(const uint8_t* _
         h = dh;
         __syncthreads();
     }
+}
+
+template <int K>
+cudaError_t launch_chain(const goofy_gpu_level* levels, uint32_t i, cudaStream_t stream)
+{
+    MipLevels<chain_levels(K)> out{};
+    for (int l = 0; l < chain_levels(K); ++l) {
+        out.data[l] = static_cast<uint8_t*>(levels[i + l].data);
+        out.pitch[l] = levels[i + l].stride;
+    }
+    const goofy_gpu_level& up = levels[i - 1];
+    const uint32_t sx = up.width / (64u * K), sy = up.height / (64u * K);
+    return goofy_gpu::launch_pdl(mip_chain_kernel<K>, dim3(sx * sy * chain_cluster(K)), dim3(256 * chain_tiles(K)), 0,
+                                 stream, static_cast<const uint8_t*>(up.data), (size_t)up.stride, sx, out);
 }
 
 bool pow2(uint32_t v) { return v && !(v & (v - 1)); }
@@ -273,6 +355,11 @@ GOOFY_EXPORT int goofy_gpu_generate_mips(const void* src, uint32_t width, uint32
         // levels from here on that halve both axes (an axis at 4 stays 4)
         uint32_t both = 0;
         for (uint32_t w = up.width, h = up.height; i + both < n && w > 4 && h > 4; w /= 2, h /= 2) ++both;
+        const bool vec16 = reinterpret_cast<uintptr_t>(up.data) % 16 == 0 && up.stride % 16 == 0;
+        if (vec16 && both == n - i && (both == 7 || both == 8)) {
+            GOOFY_CUDA_TRY(both == 7 ? launch_chain<2>(levels, i, st) : launch_chain<4>(levels, i, st));
+            break;
+        }
         uint32_t f = log2u(up.width < up.height ? up.width : up.height);
         f = f < both ? f : both;
         f = f < 6 ? f : 6;
@@ -291,7 +378,7 @@ GOOFY_EXPORT int goofy_gpu_generate_mips(const void* src, uint32_t width, uint32
                                                  up.height, n - i, to));
             break;
         }
-        if (f >= 2 && reinterpret_cast<uintptr_t>(up.data) % 16 == 0 && up.stride % 16 == 0) {
+        if (f >= 2 && vec16) {
             MipOut mo{};
             for (uint32_t l = 0; l < f; ++l) {
                 mo.data[l] = static_cast<uint8_t*>(levels[i + l].data);
