@@ -7,10 +7,16 @@
 namespace goofy_gpu {
 
 // Source pixels are read exactly once: 128-bit loads that skip L1.
+//
+// These loads are volatile and not .nc: kernels issue them behind pdl_wait(),
+// and the compiler may move an asm without a memory operand, and the assembler
+// a load of constant memory (.nc, __ldg), ahead of that wait, where the data
+// is still the previous kernel's to write (seen with .nc loads in a grid of two
+// blocks a thread).
 __device__ __forceinline__ uint4 ld_once16(const uint8_t* p)
 {
     uint4 v;
-    asm("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"
+    asm volatile("ld.global.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"
         : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
         : "l"(p));
     return v;
@@ -19,7 +25,7 @@ __device__ __forceinline__ uint4 ld_once16(const uint8_t* p)
 __device__ __forceinline__ uint32_t ld_once4(const uint8_t* p)
 {
     uint32_t v;
-    asm("ld.global.nc.L1::no_allocate.u32 %0, [%1];" : "=r"(v) : "l"(p));
+    asm volatile("ld.global.L1::no_allocate.u32 %0, [%1];" : "=r"(v) : "l"(p));
     return v;
 }
 
@@ -27,7 +33,7 @@ __device__ __forceinline__ uint32_t ld_once4(const uint8_t* p)
 __device__ __forceinline__ uint2 load_block8(const uint8_t* p)
 {
     uint2 v;
-    asm("ld.global.nc.L1::no_allocate.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
+    asm volatile("ld.global.L1::no_allocate.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
     return v;
 }
 
@@ -35,6 +41,30 @@ __device__ __forceinline__ uint2 load_block8(const uint8_t* p)
 __device__ __forceinline__ void st_stream8(uint8_t* p, uint2 v)
 {
     asm volatile("st.global.cs.v2.u32 [%0], {%1, %2};" ::"l"(p), "r"(v.x), "r"(v.y) : "memory");
+}
+
+// The same for rows that the next kernel reads again.  Behind the loads above it
+// finds less of them in L2 (a 4096^2 texture: mips, then all levels encoded,
+// 32.4 us with those, 29.7 with these).
+__device__ __forceinline__ uint4 ld_keep16(const uint8_t* p)
+{
+    uint4 v;
+    asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+}
+
+__device__ __forceinline__ uint2 ld_keep8(const uint8_t* p)
+{
+    uint2 v;
+    asm volatile("ld.global.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
+    return v;
+}
+
+__device__ __forceinline__ uint32_t ld_keep4(const uint8_t* p)
+{
+    uint32_t v;
+    asm volatile("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(p));
+    return v;
 }
 
 // 16 pixel words of the block at `p`: 16-byte aligned rows use one vector load
@@ -57,6 +87,9 @@ __device__ __forceinline__ void load_block_rows(const uint8_t* p, size_t stride,
             for (int x = 0; x < 4; ++x) w[4 * y + x] = ld_once4(p + (size_t)y * stride + 4 * x);
     }
 }
+
+// Asks L2 for the line at p.  A hint: L2 stays coherent with every later write to it.
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
 // n / d for n < 2^32 with magic = floor((2^32 - 1) / d): the estimate is low by
 // at most one, so a single correction makes it exact.
