@@ -13,12 +13,13 @@
 //
 // Up to about two thousand images, the descriptors are the kernel's parameter
 // instead (encode_batch_params): no upload and no counter to zero ahead of
-// the kernel, units sized to the work.  A call (us), uploaded / as parameter:
-// 24 tiles of 128x128 12.3 / 2.8, a 2048^2 mip chain 12 / 4, the first 20
-// textures of the mixed batch 19.2 / 9.2, 100 53.2 / 40.3 (floor 35.5 at 4.5
-// B/px of measured HBM), 380 (993 images) 148 / 137 (134), 600 (two launches)
-// 201 / 195.  Each further launch drains the GPU once, about 4 us: with 1000
-// textures (three launches, 2642 images) 323 against 317-320 us uploaded.
+// the kernel, units sized to the work.  A call (us), uploaded / as parameter
+// (both before the prefetches below) / now: 24 tiles of 128x128 12.3 / 2.8 / 2.8,
+// a 2048^2 mip chain 12 / 4 / 4, the first 20 textures of the mixed batch 19.2 / 9.2
+// / 8.4, 100 53.2 / 40.3 / 37.4 (floor 35.5 at 4.5 B/px of measured HBM), 380 (993
+// images) 148 / 137 / 128 (134), 600 (two launches) 201 / 195 / 182.  Each further
+// launch drains the GPU once, about 4 us: with 1000 textures (three launches,
+// 2642 images) 323 against 317-320 uploaded, which takes 304 now (306).
 #include <cuda_runtime.h>
 
 #include "batch.h"
@@ -28,29 +29,52 @@
 
 namespace goofy_gpu {
 
-// Encodes blocks [first, last) of one image, 32 * BPT at a time.
+// This lane's blocks of the step at b0: their addresses, and (PREFETCH) L2
+// asked for their lines, every eighth lane's block being 128 bytes on.  Blocks
+// past the unit's last are the last.
+template <int BPT>
+__device__ __forceinline__ void step_addresses(const BatchImage& im, uint32_t b0, uint32_t last, uint32_t lane,
+                                               bool prefetch, const uint8_t* (&p)[BPT])
+{
+#pragma unroll
+    for (int j = 0; j < BPT; ++j) {
+        uint32_t bx;
+        const uint32_t by = div_magic(min(b0 + lane + 32u * j, last - 1u), im.bw, im.bw_magic, bx);
+        p[j] = im.src + (size_t)by * 4u * im.stride + 16u * (size_t)bx;
+        if (prefetch && !(lane & 7u)) {
+#pragma unroll
+            for (int y = 0; y < 4; ++y) prefetch_l2(p[j] + (size_t)y * im.stride);
+        }
+    }
+}
+
+// Encodes blocks [first, last) of one image, 32 * BPT at a time, `p` being the
+// first step's addresses.  While a step waits for its rows and encodes them,
+// the next step's are on their way to L2: a warp's own steps are a serial
+// chain, and memory latency is most of each.  Whole calls without / with (us):
+// 1000 textures 319 / 304, 600 197 / 182, 380 139 / 128, 100 40.3 / 37.4.
+// Loading the next step's words into registers instead leaves too few warps
+// (1000 textures 344).
 template <int BPT>
 __device__ __forceinline__ void encode_unit(const BatchImage& im, uint32_t first, uint32_t last, uint32_t lane,
-                                            const uint8_t* ctrl_lut)
+                                            const uint8_t* (&p)[BPT], const uint8_t* ctrl_lut)
 {
     const bool vec16 = im.vec16 != 0;
     for (uint32_t b0 = first; b0 < last; b0 += 32u * BPT) {
         uint32_t w[BPT][16];
-        uint32_t blk[BPT];
+        const uint8_t* n[BPT];  // asked for ahead of this step's loads (behind them: 2 us more on 600 textures)
+        if (b0 + 32u * BPT < last) step_addresses<BPT>(im, b0 + 32u * BPT, last, lane, true, n);
 #pragma unroll
         for (int j = 0; j < BPT; ++j) {
-            blk[j] = b0 + lane + 32u * j;
-            if (blk[j] < last) {
-                uint32_t bx;
-                const uint32_t by = div_magic(blk[j], im.bw, im.bw_magic, bx);
-                load_block_rows(im.src + (size_t)by * 4u * im.stride + 16u * (size_t)bx, im.stride, vec16, w[j]);
-            }
+            if (b0 + lane + 32u * j < last) load_block_rows(p[j], im.stride, vec16, w[j]);
+            p[j] = n[j];
         }
 #pragma unroll
         for (int j = 0; j < BPT; ++j) {
-            if (blk[j] < last) {
+            const uint32_t b = b0 + lane + 32u * j;
+            if (b < last) {
                 const uint2 e = im.codec == kBC1 ? encode_bc1(w[j]) : encode_etc1s(w[j], ctrl_lut);
-                st_stream8(im.dst + 8u * (size_t)blk[j], e);
+                st_stream8(im.dst + 8u * (size_t)b, e);
             }
         }
     }
@@ -73,8 +97,10 @@ __global__ void __launch_bounds__(512) encode_batch_kernel(const BatchImage* __r
         if (u >= total_units) return;
         const uint32_t ii = find_image(first_unit, n_images, u);
         const BatchImage im = images[ii];
-        const uint32_t first = (u - im.first_unit) * unit_blocks;
-        encode_unit<BPT>(im, first, min(first + unit_blocks, im.bw * im.bh), lane, ctrl_lut);
+        const uint32_t first = (u - im.first_unit) * unit_blocks, last = min(first + unit_blocks, im.bw * im.bh);
+        const uint8_t* p[BPT];
+        step_addresses<BPT>(im, first, last, lane, false, p);
+        encode_unit<BPT>(im, first, last, lane, p, ctrl_lut);
     }
 }
 
@@ -116,8 +142,13 @@ __global__ void __launch_bounds__(512) encode_batch_params(const __grid_constant
     im.codec = p.codec();
     im.vec16 = p.vec16();
     const uint32_t unit = (32u * BPT) << p.unit_class(), first = (u - p.first_unit) * unit;
+    const uint32_t last = min(first + unit, im.bw * im.bh), lane = threadIdx.x & 31u;
+    // the first step's rows, while the previous kernel drains (20 textures 9.2 / 8.3 us); nothing
+    // of them enters the SM before the wait
+    const uint8_t* rows[BPT];
+    step_addresses<BPT>(im, first, last, lane, true, rows);
     pdl_wait();  // no global memory access before the previous kernel in the stream is done
-    encode_unit<BPT>(im, first, min(first + unit, im.bw * im.bh), threadIdx.x & 31u, ctrl_lut);
+    encode_unit<BPT>(im, first, last, lane, rows, ctrl_lut);
 }
 
 int batch_resident_ctas(uint32_t threads, uint32_t bpt, uint32_t pipeline)
