@@ -303,7 +303,7 @@ int compress_host_impl(int codec, uint8_t* dst, const uint8_t* src, uint32_t wid
             if (t.persistent == 2) t = Tile{256, 1, 0};
             CUDA_TRY(goofy_gpu::launch_image(codec, static_cast<const uint8_t*>(dsrc), stride,
                                              static_cast<uint8_t*>(ddst), width, height, t, access, hp.stream[0],
-                                             static_cast<uint8_t*>(ddst2)));
+                                             static_cast<uint8_t*>(ddst2), false));
             CUDA_TRY(cudaStreamSynchronize(hp.stream[0]));
             return GOOFY_OK;
         }

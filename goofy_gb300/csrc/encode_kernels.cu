@@ -35,6 +35,15 @@ __device__ __forceinline__ void load_block(const uint8_t* p, size_t stride, uint
     load_block_rows(p, stride, ACCESS == SrcAccess::kVec16, w);
 }
 
+// The first pixel of block b of the image in row-major order.
+__device__ __forceinline__ const uint8_t* block_address(const uint8_t* src, size_t stride, uint32_t bw,
+                                                        uint32_t bw_magic, uint32_t b)
+{
+    uint32_t bx;
+    const uint32_t by = div_magic(b, bw, bw_magic, bx);
+    return src + (size_t)by * 4u * stride + 16u * (size_t)bx;
+}
+
 // Loads this lane's blocks of segment `seg`: blocks b0, b0 + 32, ... of the
 // image in row-major order (b0 returned), so a segment runs on from one block
 // row into the next and only the image's last one is short.
@@ -47,11 +56,7 @@ __device__ __forceinline__ uint32_t load_segment(const uint8_t* __restrict__ src
 #pragma unroll
     for (int j = 0; j < BPT; ++j) {
         const uint32_t b = b0 + 32u * j;
-        if (b < total) {
-            uint32_t bx;
-            const uint32_t by = div_magic(b, bw, bw_magic, bx);
-            load_block<ACCESS>(src + (size_t)by * 4u * stride + 16u * (size_t)bx, stride, w[j]);
-        }
+        if (b < total) load_block<ACCESS>(block_address(src, stride, bw, bw_magic, b), stride, w[j]);
     }
     return b0;
 }
@@ -75,14 +80,21 @@ __device__ __forceinline__ void encode_segment(uint8_t* __restrict__ dst, uint8_
     }
 }
 
-// Persistent grid: warp-segments are dealt round-robin to the resident warps;
-// each warp loads its next segment before encoding the current one, so the
-// 64*BPT bytes per lane of the next segment are in flight during the math.
 // One segment per warp: every lane issues its 4*BPT row loads up front.
-template <int CODEC, int BPT, SrcAccess ACCESS>
-__global__ void __launch_bounds__(512) encode_image_kernel(const uint8_t* __restrict__ src, size_t stride,
-                                                           uint8_t* __restrict__ dst, uint8_t* __restrict__ dst2,
-                                                           uint32_t bw, uint32_t bw_magic, uint32_t total)
+//
+// PREFETCH (device memory): before the dependency wait, while the previous
+// kernel in the stream drains, the warp asks L2 for the lines of its rows
+// (every eighth lane's addresses are 128 bytes apart).  Only a hint: the loads
+// after the wait read what that kernel wrote.  An image whose CTAs are all
+// after the wait read what that kernel wrote.  An image whose CTAs are all
+// resident at once is then on its way to L2 before its turn comes.  Launches
+// back to back, inputs of 400 MB in all, without / with (us): 256^2 BC1 1.6 / 1.2,
+// ETC1s 1.8 / 1.3, 2048^2 BC1 4.6 / 3.7, 8192^2 BC1 45.5 / 43.  Segments of two
+// to four steps a warp, all asked for ahead, were slower at every size.
+template <int CODEC, int BPT, SrcAccess ACCESS, bool PREFETCH>
+__global__ void __launch_bounds__(512, BPT > 1 || ACCESS == SrcAccess::kWord4 || !PREFETCH ? 1 : CODEC == kBC1 ? 4 : 3)
+    encode_image_kernel(const uint8_t* __restrict__ src, size_t stride, uint8_t* __restrict__ dst,
+                        uint8_t* __restrict__ dst2, uint32_t bw, uint32_t bw_magic, uint32_t total)
 {
     pdl_launch_dependents();
     __shared__ uint8_t ctrl_lut[128];
@@ -90,14 +102,29 @@ __global__ void __launch_bounds__(512) encode_image_kernel(const uint8_t* __rest
         fill_ctrl_lut(ctrl_lut);
         __syncthreads();
     }
-    const uint32_t seg = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    const uint32_t seg = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31u;
     if (seg * (32u * BPT) >= total) return;
+    const uint32_t b0 = seg * (32u * BPT) + lane;
+    const uint8_t* p[BPT];
+#pragma unroll
+    for (int j = 0; j < BPT; ++j) {
+        p[j] = block_address(src, stride, bw, bw_magic, min(b0 + 32u * j, total - 1u));
+        if (PREFETCH && !(lane & 7u)) {
+#pragma unroll
+            for (int y = 0; y < 4; ++y) prefetch_l2(p[j] + y * stride);
+        }
+    }
     pdl_wait();
     uint32_t w[BPT][16];
-    const uint32_t b0 = load_segment<BPT, ACCESS>(src, stride, bw, bw_magic, total, seg, threadIdx.x & 31u, w);
+#pragma unroll
+    for (int j = 0; j < BPT; ++j)
+        if (b0 + 32u * j < total) load_block<ACCESS>(p[j], stride, w[j]);
     encode_segment<CODEC, BPT>(dst, dst2, total, b0, w, ctrl_lut);
 }
 
+// Persistent grid: warp-segments are dealt round-robin to the resident warps;
+// each warp loads its next segment before encoding the current one, so the
+// 64*BPT bytes per lane of the next segment are in flight during the math.
 template <int CODEC, int BPT, SrcAccess ACCESS>
 __global__ void __launch_bounds__(512) encode_image_persistent(const uint8_t* __restrict__ src, size_t stride,
                                                                uint8_t* __restrict__ dst, uint32_t bw,
@@ -148,29 +175,11 @@ static int resident_ctas(uint32_t threads)
     return n;
 }
 
-// The image kernels run with the shared-memory-heavy carveout of the
-// bulk-copy kernel (their loads bypass L1 anyway), so alternating the two
-// does not reconfigure the SMs between launches.
-template <typename K>
-static void prefer_shared(K kernel, int slot)
-{
-    static std::atomic<bool> done[64][2];
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64 || done[dev][slot].load(std::memory_order_relaxed))
-        return;
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared) !=
-        cudaSuccess)
-        cudaGetLastError();
-    done[dev][slot].store(true, std::memory_order_relaxed);
-}
-
 template <int CODEC, int BPT, SrcAccess ACCESS>
 static cudaError_t launch_t(const uint8_t* src, size_t stride, uint8_t* dst, uint8_t* dst2, uint32_t bw, uint32_t bh,
-                            uint32_t threads, bool persistent, cudaStream_t stream)
+                            uint32_t threads, bool persistent, bool prefetch, cudaStream_t stream)
 {
     constexpr bool kHasPersistent = BPT <= 2 && CODEC != kBoth;
-    prefer_shared(encode_image_kernel<CODEC, BPT, ACCESS>, 0);
-    if constexpr (kHasPersistent) prefer_shared(encode_image_persistent<CODEC, BPT, ACCESS>, 1);
     const uint32_t total = bw * bh, magic = 0xffffffffu / bw;
     const uint32_t per_cta = threads * BPT;
     uint64_t ctas = ((uint64_t)total + per_cta - 1) / per_cta;
@@ -182,19 +191,20 @@ static cudaError_t launch_t(const uint8_t* src, size_t stride, uint8_t* dst, uin
                               stream, src, stride, dst, bw, magic, total);
         }
     }
-    return launch_pdl(encode_image_kernel<CODEC, BPT, ACCESS>, dim3((unsigned)ctas), dim3(threads), 0, stream, src,
-                      stride, dst, dst2, bw, magic, total);
+    return launch_pdl(prefetch ? encode_image_kernel<CODEC, BPT, ACCESS, true>
+                               : encode_image_kernel<CODEC, BPT, ACCESS, false>,
+                      dim3((unsigned)ctas), dim3(threads), 0, stream, src, stride, dst, dst2, bw, magic, total);
 }
 
 template <int CODEC, SrcAccess ACCESS>
 static cudaError_t launch_bpt(const uint8_t* src, size_t stride, uint8_t* dst, uint8_t* dst2, uint32_t bw,
-                              uint32_t bh, Tile tile, cudaStream_t stream)
+                              uint32_t bh, Tile tile, bool prefetch, cudaStream_t stream)
 {
     switch (tile.bpt) {
-    case 1: return launch_t<CODEC, 1, ACCESS>(src, stride, dst, dst2, bw, bh, tile.threads, tile.persistent, stream);
-    case 2: return launch_t<CODEC, 2, ACCESS>(src, stride, dst, dst2, bw, bh, tile.threads, tile.persistent, stream);
+    case 1: return launch_t<CODEC, 1, ACCESS>(src, stride, dst, dst2, bw, bh, tile.threads, tile.persistent, prefetch, stream);
+    case 2: return launch_t<CODEC, 2, ACCESS>(src, stride, dst, dst2, bw, bh, tile.threads, tile.persistent, prefetch, stream);
     case 4:
-        if constexpr (CODEC != kBoth) return launch_t<CODEC, 4, ACCESS>(src, stride, dst, dst2, bw, bh, tile.threads, false, stream);
+        if constexpr (CODEC != kBoth) return launch_t<CODEC, 4, ACCESS>(src, stride, dst, dst2, bw, bh, tile.threads, false, prefetch, stream);
         return cudaErrorInvalidValue;
     default: return cudaErrorInvalidValue;
     }
@@ -202,15 +212,15 @@ static cudaError_t launch_bpt(const uint8_t* src, size_t stride, uint8_t* dst, u
 
 template <int CODEC>
 static cudaError_t launch_access(const uint8_t* src, size_t stride, uint8_t* dst, uint8_t* dst2, uint32_t bw,
-                                 uint32_t bh, Tile tile, SrcAccess access, cudaStream_t stream)
+                                 uint32_t bh, Tile tile, SrcAccess access, bool prefetch, cudaStream_t stream)
 {
     if (access == SrcAccess::kVec16)
-        return launch_bpt<CODEC, SrcAccess::kVec16>(src, stride, dst, dst2, bw, bh, tile, stream);
-    return launch_bpt<CODEC, SrcAccess::kWord4>(src, stride, dst, dst2, bw, bh, tile, stream);
+        return launch_bpt<CODEC, SrcAccess::kVec16>(src, stride, dst, dst2, bw, bh, tile, prefetch, stream);
+    return launch_bpt<CODEC, SrcAccess::kWord4>(src, stride, dst, dst2, bw, bh, tile, prefetch, stream);
 }
 
 cudaError_t launch_image(int codec, const uint8_t* src, size_t stride, uint8_t* dst, uint32_t width,
-                         uint32_t height, Tile tile, SrcAccess access, cudaStream_t stream, uint8_t* dst2)
+                         uint32_t height, Tile tile, SrcAccess access, cudaStream_t stream, uint8_t* dst2, bool prefetch)
 {
     if (!tile_valid(tile)) return cudaErrorInvalidValue;
     if (codec != kBC1 && codec != kETC1S && (codec != kBoth || !dst2)) return cudaErrorInvalidValue;
@@ -223,35 +233,48 @@ cudaError_t launch_image(int codec, const uint8_t* src, size_t stride, uint8_t* 
             const size_t out = (size_t)y * bw * 8u;
             const cudaError_t e = launch_image(codec, src + (size_t)y * 4u * stride, stride, dst + out, width,
                                                4u * std::min(band, bh - y), tile, access, stream,
-                                               dst2 ? dst2 + out : nullptr);
+                                               dst2 ? dst2 + out : nullptr, prefetch);
             if (e != cudaSuccess) return e;
         }
         return cudaSuccess;
     }
     if (tile.persistent == 2) {
         // Launches back to back over inputs of 400 MB in all (us), BC1 / ETC1s / both:
-        //                            grid 128x1           bulk copy 128x1      bulk copy 512x2
-        //   256^2     (4096 blocks)   1.6 / 1.8 / 1.7      1.6 / 1.7 / 1.7      4.1 / 4.4 / 4.7
-        //   512^2     (16384)         1.7 / 2.0 / 2.5      2.2 / 2.3 / 2.8      3.1 / 3.5 / 3.8
-        //   1024^2    (65536)         3.4 / 2.9 / 3.5      2.7 / 2.5 / 3.1      2.8 / 3.2 / 3.4
-        //   2048^2    (262144)        4.9 / 5.5 / 5.9      4.6 / 4.9 / 5.7      4.8 / 5.5 / 6.1
-        //   3840x2160 (518400)        7.7 / 9.0 / 9.6      6.7 / 7.3 / 8.4      7.1 / 8.1 / 9.0
-        //   3600x3400 (765000)       11.2 / 12.4 / 13.2   10.0 / 10.7 / 12.8    9.3 / 10.4 / 12.0
-        //   256x32768 (524288)        7.6 / 9.0 / 9.6      6.8 / 7.7 / 8.4     13.2 / 13.5 / 14.2
-        //   64x16000  (64000)         3.1 / 2.4 / 3.5      3.2 / 3.0 / 3.7     10.0 / 10.3 / 10.7
-        // A small grid is done before a pipeline has filled; one big CTA a SM leaves SMs idle in its last
-        // round on images of few units, and its one copy queue is slow on short rows.
-        constexpr uint32_t kTinyBlocks = 20000, kTinyRow = 32, kBigBlocks = 600000, kBigRow = 256;
+        //                            grid 128x1           grid 128x2           bulk copy 128x1      bulk copy 512x2
+        //   256^2     (4096 blocks)   1.2 / 1.3 / 1.35     1.3 / 1.4 / 1.5      1.6 / 1.7 / 1.7      4.1 / 4.4 / 4.7
+        //   512^2     (16384)         1.35 / 2.0 / 2.4     1.4 / 1.55 / 2.4     2.2 / 2.3 / 2.8      3.1 / 3.5 / 3.8
+        //   768^2     (36864)         1.9 / 2.25 / 2.7     2.4 / 3.0 / 3.2      2.4 / 2.5 / 2.95
+        //   1024^2    (65536)         2.25 / 2.85 / 3.1    2.8 / 3.3 / 2.8      2.6 / 2.4 / 3.05     2.8 / 3.2 / 3.4
+        //   2048x1800 (230400)        3.4 / 4.0 / 4.2      3.7 / 4.25 / 4.4     4.3 / 4.5 / 5.2
+        //   2048^2    (262144)        3.7 / 5.8 / 6.4      3.8 / 4.45 / 5.0     4.55 / 4.9 / 5.6     4.8 / 5.5 / 6.1
+        //   2400x2048 (307200)        4.1 / 6.0 / 6.8      4.15 / 5.15 / 7.2    5.0 / 5.5 / 6.2
+        //   3840x2160 (518400)        6.3 / 8.7 / 9.5      6.5 / 8.4 / 9.0      6.65 / 7.3 / 8.4     7.1 / 8.1 / 9.0
+        //   4096x3000 (768000)        8.7 / 12.0 / 13.2    9.1 / 12.3 / 12.6    9.6 / 10.4 / 12.8    9.3 / 10.4 / 12.0
+        //   4096^2    (1048576)      11.6 / 15.6 / 17.3   11.9 / 14.4 / 16.7   12.3 / 13.5 / 15.6   11.5 / 12.6 / 14.8
+        //   8192^2    (4194304)      43.0 / 54.1 / 61.0   43.7 / 49.4 / 66.8   48.6 / 47.5 / 52.8   45.8 / 45.8 / 50.1
+        //   256x32768 (524288)        6.2 / 8.6 / 9.9      7.2 / 7.7 / 8.8      6.8 / 7.8 / 8.4     13.2 / 13.5 / 14.2
+        //   64x16000  (64000)         2.1 / 2.7 / 3.2      1.8 / 2.5 / 2.35     3.2 / 3.0 / 3.7     10.0 / 10.3 / 10.7
+        // A grid whose CTAs are all resident at once has its rows prefetched while the launch before it drains; the
+        // larger of the two lets more blocks be resident.  Beyond, BC1 keeps enough warps in flight to stay at the
+        // memory's rate up to about a million blocks (8192^2: 43 to 45.7 us, the pipeline 44.9 to 45.8); the other
+        // codecs' longer blocks do not, and take the pipeline, whose copies run ahead of the codec.  One big CTA a SM
+        // leaves SMs idle in its last round on images of few units, and its one copy queue is slow on short rows.
+        constexpr uint32_t kSms = 152, kTinyBlocks = 20000, kTinyRow = 32, kBigBlocks = 600000, kBigRow = 256;
+        constexpr uint32_t kGrid1 = kSms * 12 * 128;  // resident at 128x1 (ETC1s and both; 40 registers)
+        const uint32_t grid2 = kSms * (codec == kETC1S ? 8 : 7) * 256;  // at 128x2 (62 and 72 registers)
         const uint32_t blocks = bw * bh;
-        if (blocks >= kTinyBlocks && bw >= kTinyRow) {
-            if (tile.threads == 512 && tile.bpt == 2 && (blocks < kBigBlocks || bw < kBigRow)) tile = Tile{128, 1, 2};
+        const bool by_size = tile.threads == 512 && tile.bpt == 2;
+        bool grid = blocks < kTinyBlocks || bw < kTinyRow;
+        if (by_size && access == SrcAccess::kVec16) grid |= blocks <= (codec == kBC1 ? 900000 : grid2);
+        if (!grid) {
+            if (by_size && (blocks < kBigBlocks || bw < kBigRow)) tile = Tile{128, 1, 2};
             return launch_image_tma(codec, src, stride, dst, width, height, tile, access, stream, dst2);
         }
-        tile = Tile{128, 1, 0};
+        tile = Tile{128, codec == kBC1 || blocks <= kGrid1 ? 1u : 2u, 0};
     }
-    if (codec == kBC1) return launch_access<kBC1>(src, stride, dst, nullptr, bw, bh, tile, access, stream);
-    if (codec == kETC1S) return launch_access<kETC1S>(src, stride, dst, nullptr, bw, bh, tile, access, stream);
-    return launch_access<kBoth>(src, stride, dst, dst2, bw, bh, tile, access, stream);
+    if (codec == kBC1) return launch_access<kBC1>(src, stride, dst, nullptr, bw, bh, tile, access, prefetch, stream);
+    if (codec == kETC1S) return launch_access<kETC1S>(src, stride, dst, nullptr, bw, bh, tile, access, prefetch, stream);
+    return launch_access<kBoth>(src, stride, dst, dst2, bw, bh, tile, access, prefetch, stream);
 }
 
 }  // namespace goofy_gpu
