@@ -254,23 +254,34 @@ cudaError_t launch_image(int codec, const uint8_t* src, size_t stride, uint8_t* 
         //   8192^2    (4194304)      43.0 / 54.1 / 61.0   43.7 / 49.4 / 66.8   48.6 / 47.5 / 52.8   45.8 / 45.8 / 50.1
         //   256x32768 (524288)        6.2 / 8.6 / 9.9      7.2 / 7.7 / 8.8      6.8 / 7.8 / 8.4     13.2 / 13.5 / 14.2
         //   64x16000  (64000)         2.1 / 2.7 / 3.2      1.8 / 2.5 / 2.35     3.2 / 3.0 / 3.7     10.0 / 10.3 / 10.7
-        // A grid whose CTAs are all resident at once has its rows prefetched while the launch before it drains; the
-        // larger of the two lets more blocks be resident.  Beyond, BC1 keeps enough warps in flight to stay at the
-        // memory's rate up to about a million blocks (8192^2: 43 to 45.7 us, the pipeline 44.9 to 45.8); the other
-        // codecs' longer blocks do not, and take the pipeline, whose copies run ahead of the codec.  One big CTA a SM
-        // leaves SMs idle in its last round on images of few units, and its one copy queue is slow on short rows.
+        // Word-aligned rows, BC1 / ETC1s (inputs of 400 MB; the case of inputs in L2 in brackets):
+        //   1024^2    (65536)         2.8 / 2.9            2.8 / 3.8            2.9 / 2.7
+        //   1996x1532 (191117)        3.4 / 4.7 [3.7]      4.4 / 4.6 [4.2]      4.1 / 4.6 [4.1]
+        //   2048x1800 (230400)        3.6 / 5.2            4.6 / 4.6            4.8 / 5.1
+        //   2376x2628 (390258)        5.9 / 8.2            5.7 / 7.85           6.2 / 6.75
+        //   3840x2160 (518400)        7.2 / 9.5            7.15 / 8.8           7.3 / 8.5
+        //   4096^2                   13.2 / 17.9          13.2 / 17.0          13.4 / 14.9          12.3 / 13.9
+        //
+        // A grid whose CTAs are all resident at once has its rows prefetched while the launch before it drains; two
+        // blocks a thread let more of them be resident.  Beyond, BC1 keeps enough warps in flight to stay at the
+        // memory's rate up to about a million blocks (8192^2: 43 to 45.7 us, the pipeline 44.9 to 45.8), 600,000 where
+        // each row takes four loads; the other codecs' longer blocks do not, and take the pipeline, whose copies run
+        // ahead of the codec.  One big CTA a SM leaves SMs idle in its last round on images of few units, and its one
+        // copy queue is slow on short rows.
         constexpr uint32_t kSms = 152, kTinyBlocks = 20000, kTinyRow = 32, kBigBlocks = 600000, kBigRow = 256;
-        constexpr uint32_t kGrid1 = kSms * 12 * 128;  // resident at 128x1 (ETC1s and both; 40 registers)
-        const uint32_t grid2 = kSms * (codec == kETC1S ? 8 : 7) * 256;  // at 128x2 (62 and 72 registers)
+        const bool word = access == SrcAccess::kWord4;
+        // blocks resident at 128x1 and 128x2, by the kernels' registers
+        const uint32_t grid1 = kSms * 128 * (codec == kBC1 ? 16 : !word ? 12 : codec == kETC1S ? 10 : 9);
+        const uint32_t grid2 = kSms * 256 * (codec == kETC1S ? 8 : 7);
         const uint32_t blocks = bw * bh;
         const bool by_size = tile.threads == 512 && tile.bpt == 2;
         bool grid = blocks < kTinyBlocks || bw < kTinyRow;
-        if (by_size && access == SrcAccess::kVec16) grid |= blocks <= (codec == kBC1 ? 900000 : grid2);
+        if (by_size) grid |= blocks <= (codec != kBC1 ? grid2 : word ? 600000 : 900000);
         if (!grid) {
             if (by_size && (blocks < kBigBlocks || bw < kBigRow)) tile = Tile{128, 1, 2};
             return launch_image_tma(codec, src, stride, dst, width, height, tile, access, stream, dst2);
         }
-        tile = Tile{128, codec == kBC1 || blocks <= kGrid1 ? 1u : 2u, 0};
+        tile = Tile{128, blocks <= grid1 || (codec == kBC1 && !word) ? 1u : 2u, 0};
     }
     if (codec == kBC1) return launch_access<kBC1>(src, stride, dst, nullptr, bw, bh, tile, access, prefetch, stream);
     if (codec == kETC1S) return launch_access<kETC1S>(src, stride, dst, nullptr, bw, bh, tile, access, prefetch, stream);

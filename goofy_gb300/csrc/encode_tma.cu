@@ -32,10 +32,8 @@
 // Word-aligned rows (a part of an atlas at an odd pixel offset, a padded
 // stride) take the same kernel: whole 16-byte granules are copied and the
 // shift is taken out when the words leave shared memory.  The
-// register-loading kernel reads such a block with sixteen 4-byte loads that
-// skip L1, so every 32-byte sector crosses L2 up to four times: 1996x1532
-// ETC1s 7.3-11.0 us there, 4.6 us here; 4096^2 (over 400 MB of inputs) BC1 15.8,
-// ETC1s 17.0 there with the best CTA size, 12.2 and 13.9 here.
+// register-loading kernel reads such a block with sixteen 4-byte loads
+// (launch_image has both sides' times).
 //
 // Every wait is bounded (async_copy.cuh): a stuck barrier ends the kernel with
 // a counted time-out instead of a hang, and the producer then waits (bounded)
