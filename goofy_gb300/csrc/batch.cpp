@@ -134,6 +134,7 @@ int goofy_gpu::validate_and_fill(const goofy_gpu_image* images, uint32_t count, 
     uint32_t most = 0, least = 0;
     while (most < 15 && pass << (most + 1) <= 4ull * tile.unit_blocks) ++most;
     while (least < most && pass << (least + 1) <= 128 && (pass << (least + 1)) * kResidentWarps <= left) ++least;
+    uint32_t kinds = 0;  // bit 2 * codec + (rows not 16-byte aligned)
     for (uint32_t i = 0; i < count; ++i) {
         BatchImage d;
         int rc = check_image(images[i], &d);
@@ -145,9 +146,13 @@ int goofy_gpu::validate_and_fill(const goofy_gpu_image* images, uint32_t count, 
                                   d.bh | (c >> 2) << 30, (uint32_t)units};
         if ((rc = add_units(blocks, (uint32_t)(pass << c), &units)) != GOOFY_OK) return rc;
         left -= blocks;
+        if (blocks) kinds |= 1u << (2u * d.codec + (d.vec16 ? 0u : 1u));
     }
     l->count = count;
     l->units = (uint32_t)units;
+    l->mode = kinds == 1u << (2 * GOOFY_CODEC_BC1)     ? GOOFY_CODEC_BC1
+              : kinds == 1u << (2 * GOOFY_CODEC_ETC1S) ? GOOFY_CODEC_ETC1S
+                                                       : kMixed;
     return GOOFY_OK;
 }
 

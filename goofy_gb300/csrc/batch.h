@@ -86,9 +86,13 @@ constexpr uint32_t kParamImages = 1022;
 // One launch of the work-unit kernel with its descriptors as the kernel's
 // parameter.  The launch copies 32, 256 or kParamImages entries, whichever
 // holds `count` (a smaller parameter launches faster): `images` has that room.
+// mode: the codec of all its images if their rows are all 16-byte aligned,
+// else kMixed.
+constexpr int kMixed = -1;
 struct ParamLaunch {
     ParamImage* images;
     uint32_t count, units;
+    int mode;
 };
 cudaError_t launch_batch_params(const ParamLaunch& l, const BatchTile& tile, cudaStream_t stream);
 

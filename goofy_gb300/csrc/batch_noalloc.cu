@@ -35,7 +35,7 @@ extern "C" GOOFY_EXPORT int goofy_gpu_batch_encode_noalloc(const goofy_gpu_image
     if (!images) return goofy_gpu::fail(GOOFY_ERR_INVALID, "goofy_gpu_batch_encode_noalloc: images is NULL");
     const goofy_gpu::BatchTile tile{128, 1, 256, 0};
     goofy_gpu::ParamImage table[GOOFY_NOALLOC_MAX_IMAGES];  // 8 KB of this thread's stack; the launch copies it
-    goofy_gpu::ParamLaunch l{table, 0, 0};
+    goofy_gpu::ParamLaunch l{table, 0, 0, goofy_gpu::kMixed};
     const int rc = goofy_gpu::validate_and_fill(images, count, tile, &l);
     if (rc != GOOFY_OK) return rc;  // nothing launched for an invalid batch
     GOOFY_CUDA_TRY(goofy_gpu::launch_batch_params(l, tile, static_cast<cudaStream_t>(stream)));
