@@ -58,9 +58,9 @@ __device__ __forceinline__ void step_addresses(const BatchImage& im, uint32_t b0
 //
 // MODE: the images' codec where it is one and all rows are 16-byte aligned,
 // else kMixed.
-template <int BPT, int MODE>
+template <int BPT, int MODE, typename Lut>
 __device__ __forceinline__ void encode_unit(const BatchImage& im, uint32_t first, uint32_t last, uint32_t lane,
-                                            const uint8_t* (&p)[BPT], const uint8_t* ctrl_lut)
+                                            const uint8_t* (&p)[BPT], Lut ctrl_lut)
 {
     const bool vec16 = MODE != kMixed || im.vec16 != 0;
     for (uint32_t b0 = first; b0 < last; b0 += 32u * BPT) {
@@ -103,7 +103,7 @@ __global__ void __launch_bounds__(512) encode_batch_kernel(const BatchImage* __r
         const uint32_t first = (u - im.first_unit) * unit_blocks, last = min(first + unit_blocks, im.bw * im.bh);
         const uint8_t* p[BPT];
         step_addresses<BPT>(im, first, last, lane, false, p);
-        encode_unit<BPT, kMixed>(im, first, last, lane, p, ctrl_lut);
+        encode_unit<BPT, kMixed, const uint8_t*>(im, first, last, lane, p, ctrl_lut);
     }
 }
 
@@ -126,11 +126,6 @@ __global__ void __launch_bounds__(512) encode_batch_params(const __grid_constant
                                                            uint32_t total_units)
 {
     pdl_launch_dependents();
-    __shared__ uint8_t ctrl_lut[128];
-    if constexpr (MODE != kBC1) {
-        fill_ctrl_lut(ctrl_lut);
-        __syncthreads();
-    }
     const uint32_t u = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (u >= total_units) return;
     // largest i with images[i].first_unit <= u (an image without blocks shares its successor's)
@@ -157,7 +152,7 @@ __global__ void __launch_bounds__(512) encode_batch_params(const __grid_constant
     const uint8_t* rows[BPT];
     step_addresses<BPT>(im, first, last, lane, true, rows);
     pdl_wait();  // no global memory access before the previous kernel in the stream is done
-    encode_unit<BPT, MODE>(im, first, last, lane, rows, ctrl_lut);
+    encode_unit<BPT, MODE>(im, first, last, lane, rows, NoLut{});
 }
 
 int batch_resident_ctas(uint32_t threads, uint32_t bpt, uint32_t pipeline)

@@ -61,9 +61,9 @@ __device__ __forceinline__ uint32_t load_segment(const uint8_t* __restrict__ src
     return b0;
 }
 
-template <int CODEC, int BPT>
+template <int CODEC, int BPT, typename Lut>
 __device__ __forceinline__ void encode_segment(uint8_t* __restrict__ dst, uint8_t* __restrict__ dst2, uint32_t total,
-                                               uint32_t b0, const uint32_t (&w)[BPT][16], const uint8_t* ctrl_lut)
+                                               uint32_t b0, const uint32_t (&w)[BPT][16], Lut ctrl_lut)
 {
 #pragma unroll
     for (int j = 0; j < BPT; ++j) {
@@ -97,8 +97,9 @@ __global__ void __launch_bounds__(512, BPT > 1 || ACCESS == SrcAccess::kWord4 ||
                         uint8_t* __restrict__ dst2, uint32_t bw, uint32_t bw_magic, uint32_t total)
 {
     pdl_launch_dependents();
-    __shared__ uint8_t ctrl_lut[128];
-    if constexpr (CODEC != kBC1) {
+    constexpr bool kLut = CODEC != kBC1 && BPT * (CODEC == kBoth ? 2 : 1) >= 4;  // see control_byte
+    __shared__ uint8_t ctrl_lut[kLut ? 128 : 1];
+    if constexpr (kLut) {
         fill_ctrl_lut(ctrl_lut);
         __syncthreads();
     }
@@ -119,7 +120,8 @@ __global__ void __launch_bounds__(512, BPT > 1 || ACCESS == SrcAccess::kWord4 ||
 #pragma unroll
     for (int j = 0; j < BPT; ++j)
         if (b0 + 32u * j < total) load_block<ACCESS>(p[j], stride, w[j]);
-    encode_segment<CODEC, BPT>(dst, dst2, total, b0, w, ctrl_lut);
+    if constexpr (kLut) encode_segment<CODEC, BPT, const uint8_t*>(dst, dst2, total, b0, w, ctrl_lut);
+    else encode_segment<CODEC, BPT>(dst, dst2, total, b0, w, NoLut{});
 }
 
 // Persistent grid: warp-segments are dealt round-robin to the resident warps;
@@ -146,12 +148,12 @@ __global__ void __launch_bounds__(512) encode_image_persistent(const uint8_t* __
     while (seg < segs) {
         uint32_t next = seg + warp_stride;
         if (next < segs) bb = load_segment<BPT, ACCESS>(src, stride, bw, bw_magic, total, next, lane, b);
-        encode_segment<CODEC, BPT>(dst, nullptr, total, ba, a, ctrl_lut);
+        encode_segment<CODEC, BPT, const uint8_t*>(dst, nullptr, total, ba, a, ctrl_lut);
         seg = next;
         if (seg >= segs) break;
         next = seg + warp_stride;
         if (next < segs) ba = load_segment<BPT, ACCESS>(src, stride, bw, bw_magic, total, next, lane, a);
-        encode_segment<CODEC, BPT>(dst, nullptr, total, bb, b, ctrl_lut);
+        encode_segment<CODEC, BPT, const uint8_t*>(dst, nullptr, total, bb, b, ctrl_lut);
         seg = next;
     }
 }
@@ -242,46 +244,48 @@ cudaError_t launch_image(int codec, const uint8_t* src, size_t stride, uint8_t* 
         // Launches back to back over inputs of 400 MB in all (us), BC1 / ETC1s / both:
         //                            grid 128x1           grid 128x2           bulk copy 128x1      bulk copy 512x2
         //   256^2     (4096 blocks)   1.2 / 1.3 / 1.35     1.3 / 1.4 / 1.5      1.6 / 1.7 / 1.7      4.1 / 4.4 / 4.7
-        //   512^2     (16384)         1.35 / 2.0 / 2.4     1.4 / 1.55 / 2.4     2.2 / 2.3 / 2.8      3.1 / 3.5 / 3.8
-        //   768^2     (36864)         1.9 / 2.25 / 2.7     2.4 / 3.0 / 3.2      2.4 / 2.5 / 2.95
-        //   1024^2    (65536)         2.25 / 2.85 / 3.1    2.8 / 3.3 / 2.8      2.6 / 2.4 / 3.05     2.8 / 3.2 / 3.4
-        //   2048x1800 (230400)        3.4 / 4.0 / 4.2      3.7 / 4.25 / 4.4     4.3 / 4.5 / 5.2
-        //   2048^2    (262144)        3.7 / 5.8 / 6.4      3.8 / 4.45 / 5.0     4.55 / 4.9 / 5.6     4.8 / 5.5 / 6.1
-        //   2400x2048 (307200)        4.1 / 6.0 / 6.8      4.15 / 5.15 / 7.2    5.0 / 5.5 / 6.2
-        //   3840x2160 (518400)        6.3 / 8.7 / 9.5      6.5 / 8.4 / 9.0      6.65 / 7.3 / 8.4     7.1 / 8.1 / 9.0
+        //   512^2     (16384)         1.35 / 2.0 / 2.4     1.4 / 2.4 / 2.4      2.2 / 2.3 / 2.8      3.1 / 3.5 / 3.8
+        //   1024^2    (65536)         2.25 / 2.7 / 3.05    2.8 / 2.7 / 2.8      2.6 / 2.45 / 3.05    2.8 / 3.2 / 3.4
+        //   2048x1800 (230400)        3.4 / 3.8 / 4.2      3.7 / 4.1 / 4.4      4.3 / 4.55 / 5.2
+        //   2048^2    (262144)        3.65 / 4.8 / 5.2     3.8 / 4.4 / 5.0      4.55 / 4.9 / 5.65    4.8 / 5.5 / 6.1
+        //   2400x2048 (307200)        4.1 / 5.3 / 5.8      4.15 / 6.45 / 7.15   5.0 / 5.45 / 6.3
+        //   3000x2048 (384000)         -  / 6.2 / 6.75      -  / 6.6 / 8.2       -  / 6.1 / 7.0
+        //   3840x2160 (518400)        6.25 / 8.8 / 9.7     6.5 / 8.0 / 8.95     6.65 / 7.3 / 8.4     7.1 / 8.1 / 9.0
         //   4096x3000 (768000)        8.7 / 12.0 / 13.2    9.1 / 12.3 / 12.6    9.6 / 10.4 / 12.8    9.3 / 10.4 / 12.0
-        //   4096^2    (1048576)      11.6 / 15.6 / 17.3   11.9 / 14.4 / 16.7   12.3 / 13.5 / 15.6   11.5 / 12.6 / 14.8
+        //   4096^2    (1048576)      11.6 / 14.7 / 16.5   11.9 / 14.9 / 16.6   12.3 / 13.45 / 15.55 11.5 / 12.6 / 14.7
         //   8192^2    (4194304)      43.0 / 54.1 / 61.0   43.7 / 49.4 / 66.8   48.6 / 47.5 / 52.8   45.8 / 45.8 / 50.1
         //   256x32768 (524288)        6.2 / 8.6 / 9.9      7.2 / 7.7 / 8.8      6.8 / 7.8 / 8.4     13.2 / 13.5 / 14.2
         //   64x16000  (64000)         2.1 / 2.7 / 3.2      1.8 / 2.5 / 2.35     3.2 / 3.0 / 3.7     10.0 / 10.3 / 10.7
-        // Word-aligned rows, BC1 / ETC1s (inputs of 400 MB; the case of inputs in L2 in brackets):
-        //   1024^2    (65536)         2.8 / 2.9            2.8 / 3.8            2.9 / 2.7
-        //   1996x1532 (191117)        3.4 / 4.7 [3.7]      4.4 / 4.6 [4.2]      4.1 / 4.6 [4.1]
-        //   2048x1800 (230400)        3.6 / 5.2            4.6 / 4.6            4.8 / 5.1
-        //   2376x2628 (390258)        5.9 / 8.2            5.7 / 7.85           6.2 / 6.75
+        // (With 3 inputs, mostly in L2, ETC1s and both, grid 128x1 / bulk copy: 2400x2048 4.6 / 4.9 and 5.1 / 5.35,
+        // 3000x2048 5.3 / 5.7 and 5.95 / 6.3.)  Word-aligned rows, BC1 / ETC1s, both where given:
+        //   1024^2    (65536)         2.8 / 2.9 / 3.0      2.8 / 4.0 / 3.6      2.9 / 2.75 / 3.3
+        //   1996x1532 (191117)        3.4 / 4.4 / 4.6      4.4 / 4.7 / 4.1      4.1 / 4.6 / 5.1
+        //   2048x1800 (230400)        3.6 / 4.85 / 5.1     4.6 / 4.7 / 4.8      4.8 / 5.1 / 5.6
+        //   2376x2628 (390258)        5.9 / 7.4 / 7.85     5.7 / 7.45 / 7.9     6.2 / 6.75 / 7.8
         //   3840x2160 (518400)        7.2 / 9.5            7.15 / 8.8           7.3 / 8.5
         //   4096^2                   13.2 / 17.9          13.2 / 17.0          13.4 / 14.9          12.3 / 13.9
         //
         // A grid whose CTAs are all resident at once has its rows prefetched while the launch before it drains; two
-        // blocks a thread let more of them be resident.  Beyond, BC1 keeps enough warps in flight to stay at the
+        // blocks a thread let a few more of them be resident.  Beyond, BC1 keeps enough warps in flight to stay at the
         // memory's rate up to about a million blocks (8192^2: 43 to 45.7 us, the pipeline 44.9 to 45.8), 600,000 where
-        // each row takes four loads; the other codecs' longer blocks do not, and take the pipeline, whose copies run
-        // ahead of the codec.  One big CTA a SM leaves SMs idle in its last round on images of few units, and its one
-        // copy queue is slow on short rows.
+        // each row takes four loads; the other codecs' longer blocks do not, and from 1.7 waves on take the pipeline,
+        // whose copies run ahead of the codec.  One big CTA a SM leaves SMs idle in its last round on images of few
+        // units, and its one copy queue is slow on short rows.
         constexpr uint32_t kSms = 152, kTinyBlocks = 20000, kTinyRow = 32, kBigBlocks = 600000, kBigRow = 256;
         const bool word = access == SrcAccess::kWord4;
         // blocks resident at 128x1 and 128x2, by the kernels' registers
         const uint32_t grid1 = kSms * 128 * (codec == kBC1 ? 16 : !word ? 12 : codec == kETC1S ? 10 : 9);
-        const uint32_t grid2 = kSms * 256 * (codec == kETC1S ? 8 : 7);
+        const uint32_t grid2 = kSms * 256 * (word && codec == kETC1S ? 8 : 7);
         const uint32_t blocks = bw * bh;
         const bool by_size = tile.threads == 512 && tile.bpt == 2;
         bool grid = blocks < kTinyBlocks || bw < kTinyRow;
-        if (by_size) grid |= blocks <= (codec != kBC1 ? grid2 : word ? 600000 : 900000);
+        if (by_size) grid |= blocks <= (codec == kBC1 ? (word ? 600000 : 900000) : word ? grid2 : 400000);
         if (!grid) {
             if (by_size && (blocks < kBigBlocks || bw < kBigRow)) tile = Tile{128, 1, 2};
             return launch_image_tma(codec, src, stride, dst, width, height, tile, access, stream, dst2);
         }
-        tile = Tile{128, blocks <= grid1 || (codec == kBC1 && !word) ? 1u : 2u, 0};
+        const bool two = blocks > grid1 && (word || (codec != kBC1 && blocks <= grid2));
+        tile = Tile{128, two ? 2u : 1u, 0};
     }
     if (codec == kBC1) return launch_access<kBC1>(src, stride, dst, nullptr, bw, bh, tile, access, prefetch, stream);
     if (codec == kETC1S) return launch_access<kETC1S>(src, stride, dst, nullptr, bw, bh, tile, access, prefetch, stream);

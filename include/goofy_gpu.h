@@ -142,9 +142,9 @@ typedef struct goofy_gpu_tile {
                                  *    shared-memory ring with bulk async copies (1, 2 blocks per
                                  *    thread).  Images of under 20,000 blocks or 32 blocks a row run
                                  *    shape 0.  512 x 2 leaves the choice to the image: shape 0 up
-                                 *    to the blocks that are resident at once (BC1: up to 900,000,
-                                 *    word-aligned 600,000), then 128 x 1 here, 512 x 2 for large
-                                 *    images; word-aligned sources run 128 x 1 and 512 x 2 only */
+                                 *    to 400,000 blocks (BC1 900,000; word-aligned 311,296 and
+                                 *    600,000), then 128 x 1 here, 512 x 2 for large images;
+                                 *    word-aligned sources run 128 x 1 and 512 x 2 only */
 } goofy_gpu_tile;
 
 /* Get / set the tile the image kernels launch with, per codec

@@ -15,7 +15,11 @@ pytestmark = pytest.mark.gpu
 # (width, height, extra stride bytes): blocks = width / 4 * height / 4
 SIZES = [
     (2048, 2128, 0), (2048, 2132, 16),   # 272,384 and 272,896 blocks
-    (2048, 2432, 0), (2052, 2432, 32),   # 311,296 and 311,904
+    (2048, 1824, 0), (2048, 1828, 16),   # 233,472 and 233,984
+    (2500, 2560, 0), (2500, 2564, 16),   # 400,000 and 400,625
+    (2048, 2432, 4), (2048, 2436, 12),   # 311,296 and 311,808, word-aligned
+    (1216, 2560, 4), (1216, 2564, 20),   # 194,560 and 194,864
+    (2500, 3840, 4), (2500, 3844, 4),    # 600,000 and 600,625
     (3000, 4800, 0), (3000, 4804, 16),   # 900,000 and 900,750
     (3700, 4100, 48),                    # 948,125, 925 blocks a row
     (4, 4, 0), (1024, 4, 0), (1028, 4, 0), (508, 516, 0), (120, 43000, 0),
