@@ -193,7 +193,7 @@ static cudaError_t launch_t(const uint8_t* src, size_t stride, uint8_t* dst, uin
                               stream, src, stride, dst, bw, magic, total);
         }
     }
-    return launch_pdl(prefetch ? encode_image_kernel<CODEC, BPT, ACCESS, true>
+    return launch_pdl(prefetch ? encode_image_kernel<CODEC, BPT, ACCESS, (BPT <= 2)>
                                : encode_image_kernel<CODEC, BPT, ACCESS, false>,
                       dim3((unsigned)ctas), dim3(threads), 0, stream, src, stride, dst, dst2, bw, magic, total);
 }
@@ -286,6 +286,11 @@ cudaError_t launch_image(int codec, const uint8_t* src, size_t stride, uint8_t* 
         }
         const bool two = blocks > grid1 && (word || (codec != kBC1 && blocks <= grid2));
         tile = Tile{128, two ? 2u : 1u, 0};
+    } else {
+        // A grid asked for by its shape stays without: on images far larger than the GPU holds at once the early
+        // requests gain little, and next to an ETC1s pipeline launch they cost (8192^2, both codecs in turn: 89-90.6
+        // us, both on the pipeline 87).
+        prefetch = false;
     }
     if (codec == kBC1) return launch_access<kBC1>(src, stride, dst, nullptr, bw, bh, tile, access, prefetch, stream);
     if (codec == kETC1S) return launch_access<kETC1S>(src, stride, dst, nullptr, bw, bh, tile, access, prefetch, stream);
