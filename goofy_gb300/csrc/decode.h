@@ -14,14 +14,13 @@ cudaError_t launch_decode(int codec, const uint8_t* blocks, uint32_t width, uint
 
 // Where the sums go when the launch is their only user (`sums` and *finished
 // zero before it): the last CTA to finish writes the six totals to `host`
-// (mapped host memory), leaves `sums` and *finished zero for the next launch
-// and sets *flag (mapped) to `serial`, so that the host need not wait for the
-// stream.
+// (mapped host memory) and leaves `sums` and *finished zero for the next
+// launch.  A total is never kNoTotal: with that in all six before the launch,
+// the host need not wait for the stream.
+constexpr unsigned long long kNoTotal = ~0ull;
 struct ErrorResult {
     unsigned long long* host = nullptr;
     unsigned int* finished = nullptr;
-    unsigned int* flag = nullptr;
-    unsigned int serial = 0;
 };
 
 // Adds the per-channel sums of squared differences between `src` and the

@@ -119,9 +119,7 @@ __global__ void __launch_bounds__(kDecodeThreads, CODEC == kBC1 ? 4 : 3)
         }
         if (!add_block_errors<CODEC>(cur, cur_blk, pal + threadIdx.x, kDecodeThreads, e)) ++bad;
     }
-    __shared__ unsigned long long part[6][kDecodeThreads / 32];
-    const uint64_t s[6] = {e.sq[0], e.sq[1], e.sq[2], e.sq[3], bad, luma_sum_of(e)};
-    reduce_errors<kDecodeThreads>(s, part, sums, result);
+    reduce_errors<kDecodeThreads>(e, bad, sums, result);
 }
 
 // The error sums of every image of a batch (the request server's quality

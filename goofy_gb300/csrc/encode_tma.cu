@@ -447,9 +447,7 @@ __global__ void __launch_bounds__(COMPUTE + 32, BPT == 2 ? 1 : CODEC == kBC1 ? 6
             phase ^= 1u;
         }
     }
-    __shared__ unsigned long long part[6][compute_warps];
-    const uint64_t s[6] = {e.sq[0], e.sq[1], e.sq[2], e.sq[3], bad, luma_sum_of(e)};
-    reduce_errors<COMPUTE>(s, part, sums, result);
+    reduce_errors<COMPUTE>(e, bad, sums, result);
 }
 
 // ---------------------------------------------------------------------------

@@ -30,12 +30,11 @@ int check(int codec, const void* a, const void* b, uint32_t width, uint32_t heig
 // calls: the error kernel's last CTA moves its totals to `host` and clears
 // them, so a call is one launch and a short wait.  With a memset before the
 // kernel and a copy behind it a call took 31.4 us at 4096^2 BC1 from Python,
-// 29.3 us without both, 27.2 us with the completion word polled (the kernel
-// alone 13-14 us).
+// 29.3 us without both, 27.2 us with a completion word polled, 25.0 us with the
+// totals themselves polled and a shorter end of the kernel (error_reduce.cuh).
 struct Accumulators {
     unsigned long long* sums = nullptr;  // six sums and the finished-CTA count
-    unsigned long long* host = nullptr;  // mapped: six totals and the completion word
-    uint32_t serial = 0;
+    unsigned long long* host = nullptr;  // mapped: six totals
 };
 std::mutex g_mu;
 Accumulators g_acc[64];
@@ -46,25 +45,32 @@ int accumulators(Accumulators& a)
     if (!a.sums) GOOFY_CUDA_TRY(cudaMalloc(&a.sums, 7 * sizeof(unsigned long long)));
     GOOFY_CUDA_TRY(cudaMemset(a.sums, 0, 7 * sizeof(unsigned long long)));  // on the stream of the launches
     unsigned long long* host = nullptr;
-    GOOFY_CUDA_TRY(cudaHostAlloc(&host, 7 * sizeof(unsigned long long), cudaHostAllocMapped | cudaHostAllocPortable));
-    host[6] = 0;
-    a.serial = 0;
+    GOOFY_CUDA_TRY(cudaHostAlloc(&host, 6 * sizeof(unsigned long long), cudaHostAllocMapped | cudaHostAllocPortable));
     a.host = host;
     return GOOFY_OK;
 }
 
-// Waits until the GPU has set *flag to `serial`: polls for a few milliseconds,
-// then waits for the stream, which also reports a launch that failed.  (Launch
-// and stream synchronisation of an empty kernel take 9.5 us on this GPU,
-// launch and polling 7.0.)
-cudaError_t wait_for(const unsigned int* flag, unsigned int serial, cudaStream_t stream)
+// Waits until the GPU has replaced all six kNoTotal of `host` and copies them
+// to h: polls for a few milliseconds, then waits for the stream, which also
+// reports a launch that failed.  (Launch and stream synchronisation of an
+// empty kernel take 9.5 us on this GPU, launch and polling 7.0.)
+cudaError_t wait_for(const unsigned long long* host, unsigned long long h[6], cudaStream_t stream)
 {
+    const auto read = [&] {
+        bool all = true;
+        for (int k = 0; k < 6; ++k) {
+            h[k] = __atomic_load_n(&host[k], __ATOMIC_ACQUIRE);
+            all = all && h[k] != goofy_gpu::kNoTotal;
+        }
+        return all;
+    };
     const auto t0 = std::chrono::steady_clock::now();
     do {
         for (int i = 0; i < 256; ++i)
-            if (__atomic_load_n(flag, __ATOMIC_ACQUIRE) == serial) return cudaSuccess;
+            if (read()) return cudaSuccess;
     } while (std::chrono::steady_clock::now() - t0 < std::chrono::milliseconds(5));
-    return cudaStreamSynchronize(stream);
+    const cudaError_t e = cudaStreamSynchronize(stream);
+    return e != cudaSuccess ? e : read() ? cudaSuccess : cudaErrorUnknown;
 }
 
 // The launch behind both forms of the measurement, arguments of check() passed.
@@ -130,11 +136,10 @@ int error_sums(int codec, const void* blocks, const void* src, uint32_t width, u
     Accumulators& a = g_acc[dev];
     if ((rc = accumulators(a)) != GOOFY_OK) return rc;
     cudaStream_t st = nullptr;
-    const goofy_gpu::ErrorResult result{a.host, reinterpret_cast<unsigned int*>(a.sums + 6),
-                                        reinterpret_cast<unsigned int*>(a.host + 6), ++a.serial};
+    const goofy_gpu::ErrorResult result{a.host, reinterpret_cast<unsigned int*>(a.sums + 6)};
+    for (int k = 0; k < 6; ++k) __atomic_store_n(&a.host[k], goofy_gpu::kNoTotal, __ATOMIC_RELEASE);
     if ((rc = block_error(codec, blocks, src, width, height, stride, a.sums, st, result)) != GOOFY_OK) return rc;
-    GOOFY_CUDA_TRY(wait_for(result.flag, result.serial, st));
-    std::copy(a.host, a.host + 6, h);
+    GOOFY_CUDA_TRY(wait_for(a.host, h, st));
     return GOOFY_OK;
 }
 
