@@ -297,13 +297,13 @@ int compress_host_impl(int codec, uint8_t* dst, const uint8_t* src, uint32_t wid
             const SrcAccess access = (sa % 16 == 0 && stride % 16 == 0) ? SrcAccess::kVec16 : SrcAccess::kWord4;
             // bulk async copies only ever read device memory: host rows go through the register-loading
             // kernel, in CTAs of 256 threads x 1 block.  Us a call, against 128 x 2: 2048^2 BC1 98.7 / 100.1, ETC1s
-            // 98.1 / 99.9 (the link alone takes 79.5), 4096^2 ETC1s 341.1 / 344.1, both 353.1 / 361.5, 256^2 ETC1s
-            // 16.0 / 16.2.
+            // 98.1 / 99.9 (96.5 and 96.4 with little L1, encode_kernels.cu; the link alone takes 79.5), 4096^2 ETC1s
+            // 341.1 / 344.1, both 353.1 / 361.5, 256^2 ETC1s 16.0 / 16.2.
             Tile t = tile_for(codec);
             if (t.persistent == 2) t = Tile{256, 1, 0};
             CUDA_TRY(goofy_gpu::launch_image(codec, static_cast<const uint8_t*>(dsrc), stride,
                                              static_cast<uint8_t*>(ddst), width, height, t, access, hp.stream[0],
-                                             static_cast<uint8_t*>(ddst2), false));
+                                             static_cast<uint8_t*>(ddst2), true));
             CUDA_TRY(cudaStreamSynchronize(hp.stream[0]));
             return GOOFY_OK;
         }

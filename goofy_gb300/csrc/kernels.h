@@ -33,11 +33,11 @@ enum class SrcAccess : int {
 // blocks at `dst`.  Only enqueues; returns the launch error, if any.  With
 // codec kBoth (block_codec.cuh) one pass writes the BC1 blocks to `dst` and
 // the ETC1s blocks to `dst2` (shapes: 1 or 2 blocks a thread; a resident
-// grid with prefetch runs as the plain grid).  `prefetch` false: the rows are
-// in host memory, nothing is asked of L2 ahead of the loads.
+// grid with prefetch runs as the plain grid).  `host_rows`: the rows are in
+// host memory (a grid's tile).
 cudaError_t launch_image(int codec, const uint8_t* src, size_t stride, uint8_t* dst, uint32_t width,
                          uint32_t height, Tile tile, SrcAccess access, cudaStream_t stream, uint8_t* dst2 = nullptr,
-                         bool prefetch = true);
+                         bool host_rows = false);
 
 // The bulk-copy pipeline kernel (tile.persistent == 2).  Word-aligned sources
 // (kWord4) run it with 512 x 2 tiles (rows of 205 blocks or more) or, for any

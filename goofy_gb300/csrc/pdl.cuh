@@ -22,21 +22,32 @@ __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepc
 // operations are visible; returns at once for a grid without the dependency.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// carveout: the launch's shared-memory share of L1 in percent, or -1 for the
+// driver's choice.
 template <typename... KArgs, typename... Args>
-cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
-                       Args... args)
+cudaError_t launch_pdl_carveout(int carveout, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
+                                cudaStream_t stream, Args... args)
 {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+    attr[1].val.sharedMemCarveout = (unsigned)carveout;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = carveout < 0 ? 1 : 2;
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+
+template <typename... KArgs, typename... Args>
+cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                       Args... args)
+{
+    return launch_pdl_carveout(-1, kernel, grid, block, smem, stream, args...);
 }
 
 }  // namespace goofy_gpu
