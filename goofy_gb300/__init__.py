@@ -481,8 +481,8 @@ class Batch:
 
 def batch_encode_noalloc(images, stream=None):
     """goofy_gpu_batch_encode_noalloc: a batch of at most NOALLOC_MAX_IMAGES
-    images encoded without any allocation (scratch in a fixed device array of
-    the library; calls sharing it must not overlap on the GPU)."""
+    images encoded without any allocation and without device scratch, in one
+    launch; calls may overlap on any streams."""
     arr = images if isinstance(images, ctypes.Array) else images_array(images)
     return lib().goofy_gpu_batch_encode_noalloc(arr, len(arr), stream)
 
