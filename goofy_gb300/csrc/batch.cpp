@@ -70,7 +70,7 @@ constexpr uint32_t kParamLaunches = 2;
 
 namespace {
 
-constexpr uint64_t kResidentWarps = 152 * 64;
+constexpr uint64_t kResidentWarps = 152 * 32;
 
 // Checks one image and fills its descriptor (all zero for an empty image).
 int check_image(const goofy_gpu_image& im, BatchImage* out)
@@ -124,23 +124,30 @@ int goofy_gpu::validate_and_fill(const goofy_gpu_image* images, uint32_t count, 
 
 int goofy_gpu::validate_and_fill(const goofy_gpu_image* images, uint32_t count, const BatchTile& tile, ParamLaunch* l)
 {
-    // Guided unit sizes: an image gets the largest units that still leave one for each of the GPU's warps
-    // among the blocks from it on, so the launch ends in small ones; between one pass of a warp's lanes and
-    // four of the tile's units.  A launch that fills the GPU many times over does not go below 128 blocks,
-    // where finding a unit's image begins to cost more than an even end saves.
+    // Guided unit sizes: an image gets the largest units that still leave two for each of the warps that the
+    // kernel keeps resident among the blocks from it on, so the launch ends in small ones; between one pass of a
+    // warp's lanes and four of the tile's units.  Units of 64 blocks need leave only one: a launch of one wave
+    // gains more from its second pass's early rows than from finer units (a 2048^2 chain and its mips 10.2 / 9.7
+    // us, 20 textures 8.1 / 7.0; 256-block units in one wave cost a 4096^2 chain 29.4 / 30.0).  A launch that fills
+    // the GPU many times over does not go below 128 blocks, where finding a unit's image begins to cost more than
+    // an even end saves.
     const uint64_t pass = 32u * tile.bpt;
     uint64_t left = 0, units = 0;
     for (uint32_t i = 0; i < count; ++i) left += (uint64_t)(images[i].width / 4) * (images[i].height / 4);
+    const auto fits = [&](uint32_t c) {
+        const uint64_t unit = pass << c;
+        return unit * kResidentWarps * (unit > 64 ? 2 : 1) <= left;
+    };
     uint32_t most = 0, least = 0;
     while (most < 15 && pass << (most + 1) <= 4ull * tile.unit_blocks) ++most;
-    while (least < most && pass << (least + 1) <= 128 && (pass << (least + 1)) * kResidentWarps <= left) ++least;
+    while (least < most && pass << (least + 1) <= 128 && fits(least + 1)) ++least;
     uint32_t kinds = 0;  // bit 2 * codec + (rows not 16-byte aligned)
     for (uint32_t i = 0; i < count; ++i) {
         BatchImage d;
         int rc = check_image(images[i], &d);
         if (rc != GOOFY_OK) return rc;
         uint32_t c = most;
-        while (c > least && (pass << c) * kResidentWarps > left) --c;
+        while (c > least && !fits(c)) --c;
         const uint64_t blocks = (uint64_t)d.bw * d.bh;
         l->images[i] = ParamImage{d.src, d.dst, d.stride, d.bw | d.codec << 28 | d.vec16 << 29 | (c & 3u) << 30,
                                   d.bh | (c >> 2) << 30, (uint32_t)units};
