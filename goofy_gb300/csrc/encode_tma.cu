@@ -429,7 +429,9 @@ __global__ void __launch_bounds__(COMPUTE + 32, BPT == 2 ? 1 : CODEC == kBC1 ? 6
 #pragma unroll
         for (int j = 0; j < BPT; ++j) code[j] = next[j];
         if (first + step < total) load_codes(first + step);
-        if (!mbar_wait(&full[slot], phase, &abort_flag, &g_pipeline_timeouts)) break;
+        // All lanes give up or none: behind the loop each is needed in reduce_errors, so none may be left at the
+        // __syncwarp below while others have gone there.
+        if (!__all_sync(0xffffffffu, mbar_wait(&full[slot], phase, &abort_flag, &g_pipeline_timeouts))) break;
         const uint32_t nb = min(unit, total - first);
         uint32_t bx0 = 0, w[BPT][16];
         if constexpr (WORD) div_magic(first, bw, bw_magic, bx0);
