@@ -17,7 +17,12 @@ cudaError_t launch_decode(int codec, const uint8_t* blocks, uint32_t width, uint
 // (mapped host memory) and leaves `sums` and *finished zero for the next
 // launch.  A total is never kNoTotal: with that in all six before the launch,
 // the host need not wait for the stream.
-constexpr unsigned long long kNoTotal = ~0ull;
+//
+// Total 4 is the unsupported-block count (below 2^31) and, for every warp that
+// left blocks out because a bounded wait of the ring gave up, kGaveUp: the
+// sums are then too low, and complete() is false.
+constexpr unsigned long long kNoTotal = ~0ull, kGaveUp = 1ull << 40;
+inline bool complete(const unsigned long long totals[6]) { return totals[4] < kGaveUp; }
 struct ErrorResult {
     unsigned long long* host = nullptr;
     unsigned int* finished = nullptr;

@@ -119,7 +119,7 @@ __global__ void __launch_bounds__(kDecodeThreads, CODEC == kBC1 ? 4 : 3)
         }
         if (!add_block_errors<CODEC>(cur, cur_blk, pal + threadIdx.x, kDecodeThreads, e)) ++bad;
     }
-    reduce_errors<kDecodeThreads>(e, bad, sums, result);
+    reduce_errors<kDecodeThreads>(e, bad, false, sums, result);
 }
 
 // The error sums of every image of a batch (the request server's quality

@@ -415,6 +415,7 @@ __global__ void __launch_bounds__(COMPUTE + 32, BPT == 2 ? 1 : CODEC == kBC1 ? 6
     const uint32_t step = gridDim.x * unit;
     uint32_t first = blockIdx.x * unit, slot = 0, phase = 0, bad = 0;
     ErrorSums e{};  // at most kErrorSumBlocks blocks a thread (launch_error_tma)
+    bool gave_up = false;
     uint2 next[BPT];
     auto load_codes = [&](uint32_t at) {
 #pragma unroll
@@ -431,7 +432,10 @@ __global__ void __launch_bounds__(COMPUTE + 32, BPT == 2 ? 1 : CODEC == kBC1 ? 6
         if (first + step < total) load_codes(first + step);
         // All lanes give up or none: behind the loop each is needed in reduce_errors, so none may be left at the
         // __syncwarp below while others have gone there.
-        if (!__all_sync(0xffffffffu, mbar_wait(&full[slot], phase, &abort_flag, &g_pipeline_timeouts))) break;
+        if (!__all_sync(0xffffffffu, mbar_wait(&full[slot], phase, &abort_flag, &g_pipeline_timeouts))) {
+            gave_up = true;
+            break;
+        }
         const uint32_t nb = min(unit, total - first);
         uint32_t bx0 = 0, w[BPT][16];
         if constexpr (WORD) div_magic(first, bw, bw_magic, bx0);
@@ -449,7 +453,7 @@ __global__ void __launch_bounds__(COMPUTE + 32, BPT == 2 ? 1 : CODEC == kBC1 ? 6
             phase ^= 1u;
         }
     }
-    reduce_errors<COMPUTE>(e, bad, sums, result);
+    reduce_errors<COMPUTE>(e, bad, gave_up, sums, result);
 }
 
 // ---------------------------------------------------------------------------

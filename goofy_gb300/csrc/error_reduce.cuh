@@ -23,15 +23,16 @@ __device__ __forceinline__ unsigned long long warp_total(int32_t v)  // two's co
 
 // Called by threads 0 .. THREADS - 1 of the CTA (others may have left): sums e
 // and bad over them, adds the totals with one atomic each and, with
-// result.host, lets the last CTA of the grid hand them over (decode.h).  A
+// result.host, lets the last CTA of the grid hand them over (decode.h), with
+// a kGaveUp for each warp that `gave_up` (the same in all its lanes).  A
 // synchronous call waits for all of this after its last block, so it is kept
 // short: the luminosity sum, linear in the others, is formed from the CTA's
 // totals; one warp does everything behind the one barrier; the host polls the
 // totals themselves, so nothing is fenced for it.  (A 4096^2 BC1 call from Python
 // 27.2 us before, 25.0 now.)
 template <uint32_t THREADS>
-__device__ __forceinline__ void reduce_errors(const ErrorSums& e, uint32_t bad, unsigned long long* __restrict__ sums,
-                                              const ErrorResult& result)
+__device__ __forceinline__ void reduce_errors(const ErrorSums& e, uint32_t bad, bool gave_up,
+                                              unsigned long long* __restrict__ sums, const ErrorResult& result)
 {
     constexpr uint32_t W = THREADS / 32;
     __shared__ unsigned long long part[8][W];
@@ -40,7 +41,8 @@ __device__ __forceinline__ void reduce_errors(const ErrorSums& e, uint32_t bad, 
                                      warp_total(e.sq[1]),
                                      warp_total(e.sq[2]),
                                      warp_total(e.sq[3]),
-                                     warp_total(bad),
+                                     warp_total(bad) +
+                                         (gave_up && result.host ? kGaveUp : 0ull),
                                      warp_total((int32_t)(e.pos[0] - e.neg[0])),
                                      warp_total((int32_t)(e.pos[1] - e.neg[1])),
                                      warp_total((int32_t)(e.pos[2] - e.neg[2]))};

@@ -140,6 +140,8 @@ int error_sums(int codec, const void* blocks, const void* src, uint32_t width, u
     for (int k = 0; k < 6; ++k) __atomic_store_n(&a.host[k], goofy_gpu::kNoTotal, __ATOMIC_RELEASE);
     if ((rc = block_error(codec, blocks, src, width, height, stride, a.sums, st, result)) != GOOFY_OK) return rc;
     GOOFY_CUDA_TRY(wait_for(a.host, h, st));
+    if (!goofy_gpu::complete(h))
+        return goofy_gpu::fail(GOOFY_ERR_TIMEOUT, "quality: a bounded wait of the bulk-copy ring gave up");
     return GOOFY_OK;
 }
 

@@ -216,8 +216,8 @@ int goofy_gpu_load_tile_cache(int device);
  * the cache is read again by the next goofy_gpu_init or encode call. */
 int goofy_gpu_reset_tiles(void);
 
-/* Waits of the bulk-copy pipeline (tile mode 2) that gave up after their
- * time limit on the current device (each ends its kernel early instead of
+/* Waits of the bulk-copy pipeline (tile mode 2, and the quality measurement
+ * of large images) that gave up after their time limit on the current device (each ends its kernel early instead of
  * hanging); `reset` != 0 zeroes the count.  0 in a healthy run.  Synchronous. */
 int goofy_gpu_pipeline_timeouts(uint32_t* count, int reset);
 
@@ -247,7 +247,10 @@ int goofy_gpu_decode_device(int codec, void* rgba, uint32_t rgba_stride, const v
  * differences, [4] the unsupported-block count, [5] the sum of squared
  * luminosity differences in hundredths, (21 d2 + 72 d1 + 7 d0)^2 with dk the
  * difference of byte k -- the harness's 0.21 R + 0.72 G + 0.07 B of a pixel
- * read as a little-endian u32, exact in integers.  Asynchronous. */
+ * read as a little-endian u32, exact in integers.  Asynchronous.  Large images
+ * are read by the bulk-copy pipeline: the sums miss blocks if one of its
+ * bounded waits gave up, which goofy_gpu_pipeline_timeouts counts (the
+ * synchronous calls below return GOOFY_ERR_TIMEOUT then). */
 int goofy_gpu_block_error_device(int codec, const void* blocks, const void* src, uint32_t width, uint32_t height,
                                  uint32_t stride, uint64_t* d_sums, void* stream);
 
