@@ -1,6 +1,7 @@
 // quality.cpp -- C ABI of the GPU decoder and the encode-quality measurement
 // (the reference harness's check: decode with Src/decoder.cpp, compare with
 // getMsePsnr, Src/main.cpp:403-469).
+#include <cuda.h>  // driver types for the context queries (entry points fetched at run time)
 #include <cuda_runtime.h>
 
 #include <cfloat>
@@ -10,6 +11,7 @@
 #include <mutex>
 
 #include "../../include/goofy_gpu.h"
+#include "context_slots.h"
 #include "decode.h"
 #include "host_util.h"
 
@@ -26,7 +28,34 @@ int check(int codec, const void* a, const void* b, uint32_t width, uint32_t heig
     return 1;
 }
 
-// Accumulators of the synchronous quality calls, per device.  Zero between
+// Unique id of the calling thread's current context, 0 if it has none.
+uint64_t current_context_id()
+{
+    using GetCurrent = CUresult (*)(CUcontext*);
+    using GetId = CUresult (*)(CUcontext, unsigned long long*);
+    static GetCurrent get_current = nullptr;
+    static GetId get_id = nullptr;
+    static std::once_flag once;
+    std::call_once(once, [] {
+        void* p = nullptr;
+        cudaDriverEntryPointQueryResult q{};
+        if (cudaGetDriverEntryPointByVersion("cuCtxGetCurrent", &p, 12000, cudaEnableDefault, &q) == cudaSuccess &&
+            q == cudaDriverEntryPointSuccess)
+            get_current = reinterpret_cast<GetCurrent>(p);
+        p = nullptr;
+        if (cudaGetDriverEntryPointByVersion("cuCtxGetId", &p, 12000, cudaEnableDefault, &q) == cudaSuccess &&
+            q == cudaDriverEntryPointSuccess)
+            get_id = reinterpret_cast<GetId>(p);
+        cudaGetLastError();
+    });
+    CUcontext ctx = nullptr;
+    unsigned long long id = 0;
+    if (!get_current || !get_id || get_current(&ctx) != CUDA_SUCCESS || !ctx || get_id(ctx, &id) != CUDA_SUCCESS)
+        return 0;
+    return id;
+}
+
+// Accumulators of the synchronous quality calls, per context.  Zero between
 // calls: the error kernel's last CTA moves its totals to `host` and clears
 // them, so a call is one launch and a short wait.  With a memset before the
 // kernel and a copy behind it a call took 31.4 us at 4096^2 BC1 from Python,
@@ -37,10 +66,21 @@ struct Accumulators {
     unsigned long long* host = nullptr;  // mapped: six totals
 };
 std::mutex g_mu;
-Accumulators g_acc[64];
+goofy_gpu::ContextSlots<Accumulators, 64> g_acc;
 
-int accumulators(Accumulators& a)
+// Those of the current context, which cudaDeviceReset ends with its memory:
+// pointers kept for the device would be written after that, by the host below
+// and by the kernel.
+int accumulators(Accumulators** out)
 {
+    uint64_t id = current_context_id();
+    if (id == 0) {
+        GOOFY_CUDA_TRY(cudaFree(nullptr));  // makes the device's primary context current
+        id = current_context_id();
+    }
+    if (id == 0) return goofy_gpu::fail(GOOFY_ERR_CUDA, "quality: the driver names no current context");
+    Accumulators& a = g_acc.at(id);
+    *out = &a;
     if (a.host) return GOOFY_OK;
     if (!a.sums) GOOFY_CUDA_TRY(cudaMalloc(&a.sums, 7 * sizeof(unsigned long long)));
     GOOFY_CUDA_TRY(cudaMemset(a.sums, 0, 7 * sizeof(unsigned long long)));  // on the stream of the launches
@@ -129,12 +169,10 @@ int error_sums(int codec, const void* blocks, const void* src, uint32_t width, u
 {
     int rc = check(codec, blocks, src, width, height);
     if (rc <= 0) return rc == GOOFY_OK ? GOOFY_ERR_INVALID : rc;
-    int dev = 0;
-    GOOFY_CUDA_TRY(cudaGetDevice(&dev));
-    if (dev < 0 || dev >= 64) return GOOFY_ERR_NO_DEVICE;
     std::lock_guard<std::mutex> lk(g_mu);
-    Accumulators& a = g_acc[dev];
-    if ((rc = accumulators(a)) != GOOFY_OK) return rc;
+    Accumulators* acc = nullptr;
+    if ((rc = accumulators(&acc)) != GOOFY_OK) return rc;
+    const Accumulators& a = *acc;
     cudaStream_t st = nullptr;
     const goofy_gpu::ErrorResult result{a.host, reinterpret_cast<unsigned int*>(a.sums + 6)};
     for (int k = 0; k < 6; ++k) __atomic_store_n(&a.host[k], goofy_gpu::kNoTotal, __ATOMIC_RELEASE);
