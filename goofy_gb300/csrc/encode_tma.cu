@@ -430,10 +430,11 @@ __global__ void __launch_bounds__(COMPUTE + 32, BPT == 2 ? 1 : CODEC == kBC1 ? 6
 #pragma unroll
         for (int j = 0; j < BPT; ++j) code[j] = next[j];
         if (first + step < total) load_codes(first + step);
-        // All lanes give up or none: behind the loop each is needed in reduce_errors, so none may be left at the
-        // __syncwarp below while others have gone there.
-        if (!__all_sync(0xffffffffu, mbar_wait(&full[slot], phase, &abort_flag, &g_pipeline_timeouts))) {
+        if (!mbar_wait(&full[slot], phase, &abort_flag, &g_pipeline_timeouts)) {
+            // This lane leaves its blocks out, here and in the units that follow, but lanes of its warp whose last
+            // try succeeded still need it at the __syncwarp below.
             gave_up = true;
+            for (; first < total; first += step) __syncwarp();
             break;
         }
         const uint32_t nb = min(unit, total - first);

@@ -24,7 +24,7 @@ __device__ __forceinline__ unsigned long long warp_total(int32_t v)  // two's co
 // Called by threads 0 .. THREADS - 1 of the CTA (others may have left): sums e
 // and bad over them, adds the totals with one atomic each and, with
 // result.host, lets the last CTA of the grid hand them over (decode.h), with
-// a kGaveUp for each warp that `gave_up` (the same in all its lanes).  A
+// a kGaveUp for each warp with a lane that `gave_up`.  A
 // synchronous call waits for all of this after its last block, so it is kept
 // short: the luminosity sum, linear in the others, is formed from the CTA's
 // totals; one warp does everything behind the one barrier; the host polls the
@@ -42,7 +42,7 @@ __device__ __forceinline__ void reduce_errors(const ErrorSums& e, uint32_t bad, 
                                      warp_total(e.sq[2]),
                                      warp_total(e.sq[3]),
                                      warp_total(bad) +
-                                         (gave_up && result.host ? kGaveUp : 0ull),
+                                         (__any_sync(0xffffffffu, gave_up) && result.host ? kGaveUp : 0ull),
                                      warp_total((int32_t)(e.pos[0] - e.neg[0])),
                                      warp_total((int32_t)(e.pos[1] - e.neg[1])),
                                      warp_total((int32_t)(e.pos[2] - e.neg[2]))};
