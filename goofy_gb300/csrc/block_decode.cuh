@@ -7,8 +7,8 @@
 // (differential, zero deltas, one table: every block this encoder writes)
 // hold their palette as one word per channel, colour k in byte k, and a row's
 // four slots as the selector of a byte permute: one instruction gives a
-// channel of four pixels.  Other ETC1 blocks put 4 RGBA words per sub-block
-// (8) into a per-thread column of a store (shared memory on the device: entry
+// channel of four pixels.  Other ETC1 blocks, decoded to pixels, put 4 RGBA
+// words per sub-block (8) into a per-thread column of a store (shared memory on the device: entry
 // k of thread t at store[k * stride + t], bank-conflict free) and take each
 // pixel with one indexed load.  (All blocks through the store: decoding took
 // 1-4 % longer, 4096^2 ETC1s 12.7 against 12.3 us.)
@@ -169,6 +169,28 @@ GOOFY_FN void etc1s_palette(uint32_t w0, uint32_t (&pal)[4])
     pal[2] = etc1s_channel((e >> 8) & 0xffu, sl);
     pal[3] = 0xffffffffu;
 }
+
+// Palette words R, G, B of both sub-blocks of any ETC1 block, and their alpha.
+// False, and zeros, for an unsupported one.
+GOOFY_FN bool etc1_palettes(uint32_t w0, uint32_t (&pal)[3], uint32_t (&pal1)[3], uint32_t& alpha)
+{
+    uint32_t b0, b1;
+    const bool ok = etc1_bases(w0, b0, b1);
+    const uint32_t t0 = (w0 >> 5) & 7u, t1 = (w0 >> 2) & 7u;
+    const uint32_t sl0 = (uint32_t)etc1_small(t0) | (uint32_t)etc1_large(t0) << 16;
+    const uint32_t sl1 = (uint32_t)etc1_small(t1) | (uint32_t)etc1_large(t1) << 16;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        pal[k] = ok ? etc1s_channel((b0 >> (8 * k)) & 0xffu, sl0) : 0u;
+        pal1[k] = ok ? etc1s_channel((b1 >> (8 * k)) & 0xffu, sl1) : 0u;
+    }
+    alpha = ok ? 0xffffffffu : 0u;
+    return ok;
+}
+
+// Which nibbles of row y's selector pick from the second sub-block (4 added):
+// the lower rows with flip, the right columns without.
+GOOFY_FN uint32_t etc1_half(uint32_t w0, int y) { return (w0 & 1u) ? (y < 2 ? 0u : 0x4444u) : 0x4400u; }
 
 // Selector (low four nibbles) of pixel row y: pixel (x, y) keeps its low bit
 // at 4x + y of the index word and its high bit at 16 + 4x + y, nibble x.

@@ -89,7 +89,6 @@ __global__ void __launch_bounds__(kDecodeThreads, CODEC == kBC1 ? 4 : 3)
                        size_t stride, bool vec16, unsigned long long* __restrict__ sums, ErrorResult result)
 {
     pdl_launch_dependents();
-    __shared__ uint32_t pal[CODEC == kBC1 ? 1 : 8 * kDecodeThreads];  // for ETC1 blocks of other shapes than ETC1s
     const uint32_t bw_magic = 0xffffffffu / bw;
     ErrorSums e{};  // at most kErrorSumBlocks blocks a thread (launch_block_error)
     uint32_t bad = 0;
@@ -117,7 +116,7 @@ __global__ void __launch_bounds__(kDecodeThreads, CODEC == kBC1 ? 4 : 3)
             load_block_rows(src + (size_t)by * 4u * stride + 16u * (size_t)bx, stride, vec16, w);
             blk = load_block8(blocks + 8u * (size_t)(i + step));
         }
-        if (!add_block_errors<CODEC>(cur, cur_blk, pal + threadIdx.x, kDecodeThreads, e)) ++bad;
+        if (!add_block_errors<CODEC>(cur, cur_blk, e)) ++bad;
     }
     reduce_errors<kDecodeThreads>(e, bad, false, sums, result);
 }
@@ -133,7 +132,6 @@ __global__ void __launch_bounds__(kDecodeThreads) quality_batch_kernel(const Bat
                                                             uint32_t* __restrict__ work_counter,
                                                             unsigned long long* __restrict__ sums)
 {
-    __shared__ uint32_t pal[8 * kDecodeThreads];
     const uint32_t lane = threadIdx.x & 31u;
     for (;;) {
         uint32_t u = 0;
@@ -151,9 +149,7 @@ __global__ void __launch_bounds__(kDecodeThreads) quality_batch_kernel(const Bat
             uint32_t w[16];
             const uint2 blk = load_block8(im.dst + 8u * (size_t)b);
             load_block_rows(im.src + (size_t)by * 4u * im.stride + 16u * (size_t)bx, im.stride, im.vec16 != 0, w);
-            const bool ok = im.codec == kBC1
-                                ? add_block_errors<kBC1>(w, blk, pal + threadIdx.x, kDecodeThreads, e)
-                                : add_block_errors<kETC1S>(w, blk, pal + threadIdx.x, kDecodeThreads, e);
+            const bool ok = im.codec == kBC1 ? add_block_errors<kBC1>(w, blk, e) : add_block_errors<kETC1S>(w, blk, e);
             bad += ok ? 0u : 1u;
         }
         unsigned long long t[6] = {e.sq[0], e.sq[1], e.sq[2], e.sq[3], bad, luma_sum_of(e)};

@@ -397,7 +397,6 @@ __global__ void __launch_bounds__(COMPUTE + 32, BPT == 2 ? 1 : CODEC == kBC1 ? 6
     constexpr TmaLayout L = tma_layout(COMPUTE, BPT, WORD);
     uint64_t* full = reinterpret_cast<uint64_t*>(smem + L.stages * L.stage_bytes);
     uint64_t* empty = full + L.stages;
-    uint32_t* pal = reinterpret_cast<uint32_t*>(empty + L.stages);  // ETC1 blocks of other shapes than ETC1s
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
     const RingImage<WORD> im(src, stride, bw, bw_magic, total);
 
@@ -443,8 +442,7 @@ __global__ void __launch_bounds__(COMPUTE + 32, BPT == 2 ? 1 : CODEC == kBC1 ? 6
         load_stage<BPT, WORD, false>(smem + slot * L.stage_bytes, L.row_bytes, warp, lane, nb, bx0, bw, bw_magic, im.shift, w);
 #pragma unroll
         for (int j = 0; j < BPT; ++j)
-            if ((warp * BPT + j) * 32u + lane < nb)
-                bad += add_block_errors<CODEC>(w[j], code[j], pal + threadIdx.x, COMPUTE, e) ? 0u : 1u;
+            if ((warp * BPT + j) * 32u + lane < nb) bad += add_block_errors<CODEC>(w[j], code[j], e) ? 0u : 1u;
         // Release the stage only now (see encode_image_tma): every loaded word has gone into these sums.
         asm volatile("" ::"r"(e.sq[0]), "r"(e.sq[1]), "r"(e.sq[2]), "r"(e.sq[3]) : "memory");
         __syncwarp();
@@ -778,7 +776,7 @@ cudaError_t launch_error_t(const uint8_t* blocks, const uint8_t* src, size_t str
                            unsigned long long* sums, ErrorResult result, cudaStream_t stream)
 {
     constexpr TmaLayout L = tma_layout(COMPUTE, BPT, WORD);
-    constexpr size_t smem = (size_t)L.stages * (L.stage_bytes + 16u) + (CODEC == kBC1 ? 0u : 32u * COMPUTE);
+    constexpr size_t smem = (size_t)L.stages * (L.stage_bytes + 16u);
     const auto kernel = error_image_tma<CODEC, BPT, COMPUTE, WORD>;
     static std::atomic<int> resident[64];
     int ctas = 0;
