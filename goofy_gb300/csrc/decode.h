@@ -35,11 +35,10 @@ cudaError_t launch_block_error(int codec, const uint8_t* blocks, const uint8_t* 
                                size_t stride, bool vec16, unsigned long long* sums, cudaStream_t stream,
                                ErrorResult result = {});
 
-// The same on the bulk-copy ring (encode_tma.cu), images of 32 blocks a row and
-// more; `big`: CTAs of 512 threads x 2 blocks (rows of 205 blocks and more),
-// else 128 x 1.
+// The same on the bulk-copy ring (encode_tma.cu), for rows of 205 blocks and
+// more.
 cudaError_t launch_error_tma(int codec, const uint8_t* blocks, const uint8_t* src, uint32_t width, uint32_t height,
-                             size_t stride, bool vec16, bool big, unsigned long long* sums, ErrorResult result,
+                             size_t stride, bool vec16, unsigned long long* sums, ErrorResult result,
                              cudaStream_t stream);
 
 struct BatchImage;

@@ -79,10 +79,14 @@ __global__ void __launch_bounds__(kDecodeThreads) decode_image_kernel(const uint
     }
 }
 
-// Tiny images and narrow rows; the others take error_image_tma (encode_tma.cu).
-// Resident grid: each thread walks blocks with a grid stride, then the CTA
-// reduces and adds its six totals.  Register caps for 4 (BC1) / 3 (ETC1) CTAs
-// per SM, no spills.
+// All but large images, which take error_image_tma (encode_tma.cu).  Resident
+// grid: each thread walks blocks with a grid stride, then the CTA reduces and
+// adds its six totals.  Register caps for 4 (BC1) / 3 (ETC1) CTAs per SM, no
+// spills (ETC1 with 4: 3.9 -> 4.4 us at 1024^2).  While the previous kernel in
+// the stream drains, the first blocks' rows are asked of L2 (a hint: the loads
+// after the wait read what that kernel wrote): BC1 / ETC1s back to back over
+// 400 MB, without / with (us): 1024^2 4.4 / 4.0 and 3.9 / 3.4, 2048^2 6.75 / 5.75
+// and 6.3 / 5.2.
 template <int CODEC>
 __global__ void __launch_bounds__(kDecodeThreads, CODEC == kBC1 ? 4 : 3)
     block_error_kernel(const uint8_t* __restrict__ blocks, uint32_t bw, uint32_t nblk, const uint8_t* __restrict__ src,
@@ -92,17 +96,23 @@ __global__ void __launch_bounds__(kDecodeThreads, CODEC == kBC1 ? 4 : 3)
     const uint32_t bw_magic = 0xffffffffu / bw;
     ErrorSums e{};  // at most kErrorSumBlocks blocks a thread (launch_block_error)
     uint32_t bad = 0;
+    const uint32_t step = gridDim.x * kDecodeThreads;
+    uint32_t i = blockIdx.x * kDecodeThreads + threadIdx.x;
+    uint32_t bx0;
+    const uint32_t by0 = div_magic(min(i, nblk - 1u), bw, bw_magic, bx0);
+    const uint8_t* p0 = src + (size_t)by0 * 4u * stride + 16u * (size_t)bx0;
+    if (!(threadIdx.x & 7u)) {  // eight blocks' rows are 128 bytes, sixteen codes
+#pragma unroll
+        for (int y = 0; y < 4; ++y) prefetch_l2(p0 + (size_t)y * stride);
+        if (!(threadIdx.x & 15u)) prefetch_l2(blocks + 8u * (size_t)min(i, nblk - 1u));
+    }
     pdl_wait();
     // software pipeline: the next block's source rows and code are loaded
     // before this block is compared
-    const uint32_t step = gridDim.x * kDecodeThreads;
-    uint32_t i = blockIdx.x * kDecodeThreads + threadIdx.x;
     uint32_t w[16];
     uint2 blk = make_uint2(0, 0);
     if (i < nblk) {
-        uint32_t bx;
-        const uint32_t by = div_magic(i, bw, bw_magic, bx);
-        load_block_rows(src + (size_t)by * 4u * stride + 16u * (size_t)bx, stride, vec16, w);
+        load_block_rows(p0, stride, vec16, w);
         blk = load_block8(blocks + 8u * (size_t)i);
     }
     for (; i < nblk; i += step) {
@@ -241,13 +251,22 @@ cudaError_t launch_block_error(int codec, const uint8_t* blocks, const uint8_t* 
 {
     const uint32_t bw = width / 4, nblk = bw * (height / 4);
     if (nblk == 0) return cudaSuccess;
-    // The lines are the image encoder's (launch_image).  Launches back to back (us), this kernel / the ring, BC1
-    // and ETC1s: 2048^2 6.1 / 5.1 and 5.9 / 5.1, 4096^2 14.1 / 12.9 and 14.0 / 12.8, 8192^2 46.0 / 42.7 and 46.7 /
-    // 42.7 (floors 2.8, 11.3, 45.1 at 4.5 B/px of measured HBM: nothing is written, and reads alone run faster than
-    // the copy the floor is taken from); 1024^2 2.8 / 3.1 with the image in L2, 3.7 / 3.3 from HBM.
-    if (nblk >= 20000 && bw >= 32)
-        return launch_error_tma(codec, blocks, src, width, height, stride, vec16, nblk >= 600000 && bw >= 256, sums,
-                                result, stream);
+    // The ring keeps more bytes in flight but has to fill first and ends in an uneven round: it is for large images,
+    // and larger ones where nothing runs before or behind the launch to hide that (a synchronous call) or where it
+    // copies word-aligned rows in granules.  This kernel / the ring, BC1, us, image in L2 and from HBM:
+    //                    launches back to back              synchronous calls from Python
+    //   1024^2          3.1 / 3.2      4.0 / 3.75         13.4 / 13.7    14.0 / 14.3
+    //   2048^2          5.15 / 5.1     5.75 / 5.75        15.5 / 16.5    16.4 / 17.75
+    //   3300^2          9.7 / 9.2      9.75 / 10.0        20.2 / 20.9    20.4 / 22.2
+    //   4096^2         13.1 / 12.0    13.2 / 12.9         23.8 / 24.3    24.0 / 25.15
+    //   6000x4000      17.75 / 16.4   17.8 / 16.9         28.1 / 29.05   28.5 / 29.7
+    //   8192^2         43.2 / 40.0    44.2 / 42.6         54.0 / 52.6    55.0 / 55.5
+    //   128x65536       7.6 / 8.9      8.1 / 9.6          18.2 / 20.2    18.9 / 20.3
+    //   512x32768      13.1 / 12.6    13.2 / 13.8         23.8 / 24.8    23.85 / 25.3
+    // word-aligned 4096^2 13.2 / 14.8, 15.0 / 15.0; 6000x4000 18.3 / 19.8, 19.7 / 20.0; 8192^2 49.0 / 46.8.  ETC1s alike.
+    const bool late = result.host || !vec16;
+    if (nblk >= (late ? 2500000u : 1000000u) && bw >= 256)
+        return launch_error_tma(codec, blocks, src, width, height, stride, vec16, sums, result, stream);
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);

@@ -380,13 +380,12 @@ __global__ void __launch_bounds__(COMPUTE + 32, tma_min_ctas(BPT, COMPUTE))
 // The quality measurement on the same ring: the compute warps compare each
 // block with its rows (block_error.cuh) instead of encoding it.  A thread's
 // codes of the next unit are loaded while it works on this one.  Bound by
-// HBM at 8192^2 (42.7 us, 7.07 TB/s); with the rows loaded into registers a
-// block ahead it was short of bytes in flight (46.0 us, and 14.1 against 12.9
-// at 4096^2).  The arithmetic alone did not change that: the same sums from
-// pixels decoded through shared memory took as long.
+// HBM at 8192^2 (42.6 us, 7.09 TB/s); with the rows loaded into registers a
+// block ahead it is short of bytes in flight there (44.2 us).  Smaller images
+// do better by the registers (launch_block_error has both sides).
 // ---------------------------------------------------------------------------
 template <int CODEC, int BPT, int COMPUTE, bool WORD>
-__global__ void __launch_bounds__(COMPUTE + 32, BPT == 2 ? 1 : CODEC == kBC1 ? 6 : 5)
+__global__ void __launch_bounds__(COMPUTE + 32, 1)
     error_image_tma(const uint8_t* __restrict__ blocks, const uint8_t* __restrict__ src, size_t stride, uint32_t bw,
                     uint32_t bw_magic, uint32_t total, unsigned long long* __restrict__ sums, ErrorResult result)
 {
@@ -771,10 +770,11 @@ cudaError_t launch_image_tma(int codec, const uint8_t* src, size_t stride, uint8
 
 namespace {
 
-template <int CODEC, int BPT, int COMPUTE, bool WORD>
+template <int CODEC, bool WORD>
 cudaError_t launch_error_t(const uint8_t* blocks, const uint8_t* src, size_t stride, uint32_t bw, uint32_t bh,
                            unsigned long long* sums, ErrorResult result, cudaStream_t stream)
 {
+    constexpr int BPT = 2, COMPUTE = 512;
     constexpr TmaLayout L = tma_layout(COMPUTE, BPT, WORD);
     constexpr size_t smem = (size_t)L.stages * (L.stage_bytes + 16u);
     const auto kernel = error_image_tma<CODEC, BPT, COMPUTE, WORD>;
@@ -790,27 +790,19 @@ cudaError_t launch_error_t(const uint8_t* blocks, const uint8_t* src, size_t str
                       total, sums, result);
 }
 
-template <int CODEC, bool WORD>
-cudaError_t launch_error(const uint8_t* blocks, const uint8_t* src, size_t stride, uint32_t bw, uint32_t bh,
-                         unsigned long long* sums, ErrorResult result, bool big, cudaStream_t stream)
-{
-    return big ? launch_error_t<CODEC, 2, 512, WORD>(blocks, src, stride, bw, bh, sums, result, stream)
-               : launch_error_t<CODEC, 1, 128, WORD>(blocks, src, stride, bw, bh, sums, result, stream);
-}
-
 }  // namespace
 
 cudaError_t launch_error_tma(int codec, const uint8_t* blocks, const uint8_t* src, uint32_t width, uint32_t height,
-                             size_t stride, bool vec16, bool big, unsigned long long* sums, ErrorResult result,
+                             size_t stride, bool vec16, unsigned long long* sums, ErrorResult result,
                              cudaStream_t stream)
 {
     const uint32_t bw = width / 4, bh = height / 4;
-    if (!vec16 && !word_rows_fit(big ? 1024 : 128, bw)) return cudaErrorInvalidValue;
+    if (!vec16 && !word_rows_fit(1024, bw)) return cudaErrorInvalidValue;
     if (codec == kBC1)
-        return vec16 ? launch_error<kBC1, false>(blocks, src, stride, bw, bh, sums, result, big, stream)
-                     : launch_error<kBC1, true>(blocks, src, stride, bw, bh, sums, result, big, stream);
-    return vec16 ? launch_error<kETC1S, false>(blocks, src, stride, bw, bh, sums, result, big, stream)
-                 : launch_error<kETC1S, true>(blocks, src, stride, bw, bh, sums, result, big, stream);
+        return vec16 ? launch_error_t<kBC1, false>(blocks, src, stride, bw, bh, sums, result, stream)
+                     : launch_error_t<kBC1, true>(blocks, src, stride, bw, bh, sums, result, stream);
+    return vec16 ? launch_error_t<kETC1S, false>(blocks, src, stride, bw, bh, sums, result, stream)
+                 : launch_error_t<kETC1S, true>(blocks, src, stride, bw, bh, sums, result, stream);
 }
 
 namespace {
