@@ -142,11 +142,11 @@ int goofy_gpu::validate_and_fill(const goofy_gpu_image* images, uint32_t count, 
     while (most < 15 && pass << (most + 1) <= 4ull * tile.unit_blocks) ++most;
     while (least < most && pass << (least + 1) <= 128 && fits(least + 1)) ++least;
     uint32_t kinds = 0;  // bit 2 * codec + (rows not 16-byte aligned)
+    uint32_t c = most;   // what does not fit one image's remainder does not fit the next one's: the size only falls
     for (uint32_t i = 0; i < count; ++i) {
         BatchImage d;
         int rc = check_image(images[i], &d);
         if (rc != GOOFY_OK) return rc;
-        uint32_t c = most;
         while (c > least && !fits(c)) --c;
         const uint64_t blocks = (uint64_t)d.bw * d.bh;
         l->images[i] = ParamImage{d.src, d.dst, d.stride, d.bw | d.codec << 28 | d.vec16 << 29 | (c & 3u) << 30,
