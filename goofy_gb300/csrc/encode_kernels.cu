@@ -92,13 +92,26 @@ __device__ __forceinline__ void encode_segment(uint8_t* __restrict__ dst, uint8_
 // kernel in the stream drains, the warp asks L2 for the lines of its rows
 // (every eighth lane's addresses are 128 bytes apart).  Only a hint: the loads
 // after the wait read what that kernel wrote.  An image whose CTAs are all
-// after the wait read what that kernel wrote.  An image whose CTAs are all
 // resident at once is then on its way to L2 before its turn comes.  Launches
 // back to back, inputs of 400 MB in all, without / with (us): 256^2 BC1 1.6 / 1.2,
 // ETC1s 1.8 / 1.3, 2048^2 BC1 4.6 / 3.7, 8192^2 BC1 45.5 / 43.  Segments of two
 // to four steps a warp, all asked for ahead, were slower at every size.
+//
+// The register caps are for CTAs that fit on an SM (CTAs of 512 a cap allows).
+// Without PREFETCH, on images of more than a wave, two blocks a thread of ETC1s
+// or both codecs are held to 64: at the 66 to 73 that they take by themselves
+// an SM has one CTA of 512 threads instead of two (8192^2 ETC1s 67.8 against
+// 51.3 us, both 76.4 / 59.8) and three of 256 instead of four (53.1 / 50.5).
+// Word-aligned ETC1s takes 62 anyway and would spill.
 template <int CODEC, int BPT, SrcAccess ACCESS, bool PREFETCH>
-__global__ void __launch_bounds__(512, BPT > 1 || ACCESS == SrcAccess::kWord4 || !PREFETCH ? 1 : CODEC == kBC1 ? 4 : 3)
+constexpr int grid_min_ctas()
+{
+    if (!PREFETCH) return BPT == 2 && (CODEC == kBoth || (CODEC == kETC1S && ACCESS == SrcAccess::kVec16)) ? 2 : 1;
+    return BPT > 1 || ACCESS == SrcAccess::kWord4 ? 1 : CODEC == kBC1 ? 4 : 3;
+}
+
+template <int CODEC, int BPT, SrcAccess ACCESS, bool PREFETCH>
+__global__ void __launch_bounds__(512, (grid_min_ctas<CODEC, BPT, ACCESS, PREFETCH>()))
     encode_image_kernel(const uint8_t* __restrict__ src, size_t stride, uint8_t* __restrict__ dst,
                         uint8_t* __restrict__ dst2, uint32_t bw, uint32_t bw_magic, uint32_t total)
 {
@@ -200,7 +213,7 @@ static cudaError_t launch_t(const uint8_t* src, size_t stride, uint8_t* dst, uin
         }
     }
     return launch_pdl_carveout(rows == Rows::kHost ? 100 : -1,
-                               rows == Rows::kAhead ? encode_image_kernel<CODEC, BPT, ACCESS, (BPT <= 2)>
+                               rows == Rows::kAhead ? encode_image_kernel<CODEC, BPT, ACCESS, true>
                                                     : encode_image_kernel<CODEC, BPT, ACCESS, false>,
                                dim3((unsigned)ctas), dim3(threads), 0, stream, src, stride, dst, dst2, bw, magic, total);
 }
@@ -294,10 +307,21 @@ cudaError_t launch_image(int codec, const uint8_t* src, size_t stride, uint8_t* 
         }
         const bool two = blocks > grid1 && (word || (codec != kBC1 && blocks <= grid2));
         tile = Tile{128, two ? 2u : 1u, 0};
-        // A grid asked for by its shape does not prefetch: on images far larger than the GPU holds at once the early
-        // requests gain little, and next to an ETC1s pipeline launch they cost (8192^2, both codecs in turn: 89-90.6
-        // us, both on the pipeline 87).
         if (!host_rows) rows = Rows::kAhead;
+    } else if (tile.persistent == 0 && !host_rows) {
+        // A grid asked for by its shape has its rows prefetched as well, without / with, us, in L2 and from HBM:
+        //   128x1 BC1    2048^2 3.9 / 3.5, 4.7 / 3.8    4096^2 12.0 / 10.25, 12.1 / 10.9    6000x4000 16.1 / 18.0
+        //   128x2 ETC1s  2048^2 3.8 / 3.6, 5.4 / 4.3    4096^2 14.6 / 12.7, 14.8 / 14.2
+        //   128x4 ETC1s  2048^2 5.2 / 4.15, 6.9 / 4.9   4096^2 16.5 / 13.8, 16.6 / 15.5
+        // but not on images far larger than the GPU holds at once, where BC1 loses and, next to an ETC1s pipeline launch,
+        // the two calls do (8192^2, both codecs in turn: 89-90.6 us, both on the pipeline 87); nor on word-aligned rows
+        // (3072^2 128x1 ETC1s 9.5 / 10.4 from HBM); nor, in two blocks a thread of the longer codecs, with CTAs of which
+        // fewer fit on an SM than under the cap of the plain kernel, unless it is all one wave (256x2 ETC1s: 2048^2 5.8 / 6.3,
+        // 3072^2 9.9 / 9.6; 1024^2 both 4.6 / 3.05).
+        const uint32_t blocks = bw * bh;
+        const bool word = access == SrcAccess::kWord4, fewer = tile.bpt == 2 && codec != kBC1;
+        const uint32_t wave = 152u * 2u * tile.threads * (tile.threads == 128 ? 7u : tile.threads == 256 ? 3u : 1u);
+        if (fewer && (word || tile.threads > 128) ? blocks <= wave : !word && blocks <= 1250000u) rows = Rows::kAhead;
     }
     if (codec == kBC1) return launch_access<kBC1>(src, stride, dst, nullptr, bw, bh, tile, access, rows, stream);
     if (codec == kETC1S) return launch_access<kETC1S>(src, stride, dst, nullptr, bw, bh, tile, access, rows, stream);
