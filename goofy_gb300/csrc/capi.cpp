@@ -77,12 +77,12 @@ Tile tile_for(int codec)
     return g_tile[codec == GOOFY_CODEC_BOTH ? 2 : codec & 1];
 }
 
-// Name and SM count of a device: the key of its tile cache entries.
+// Name (with the kernels' revision) and SM count of a device: the key of its tile cache entries.
 int device_key(int dev, std::string* name, uint32_t* sms)
 {
     cudaDeviceProp p;
     CUDA_TRY(cudaGetDeviceProperties(&p, dev));
-    *name = p.name;
+    *name = goofy_gpu::tile_cache_gpu(p.name);
     *sms = (uint32_t)p.multiProcessorCount;
     return GOOFY_OK;
 }

@@ -2,13 +2,14 @@
 //
 // No reference counterpart: the reference's encoder has no launch shape to
 // tune (goofy_tc.h runs one fixed SSE2 loop).  The fastest image-kernel tile
-// differs between GB300 boxes (the register-loading BC1 grid took 39.5-51 us
+// differs between GB300 boxes (an earlier register-loading BC1 grid took 39.5-51 us
 // at 8192x8192 for the same shape), so goofy_gpu_autotune records its pick
 // here, and goofy_gpu_init / the first call of a process (the drop-in
 // included) install the recorded tiles instead of the compiled defaults.
 //
 // The file is plain text, one entry per line, '|'-separated:
 //     v1|<GPU name>|<SM count>|<codec: bc1, etc1s, both>|<threads>|<blocks a thread>|<mode>|<us>
+// The GPU name carries the kernels' revision (tile_cache_gpu).
 // '#' starts a comment line.  A line that does not parse, names a tile the
 // kernels cannot run, or belongs to another GPU model is ignored.  Writers
 // rewrite the whole file into a temporary sibling and rename it over the old
@@ -113,6 +114,8 @@ void make_parent_dirs(const std::string& path)
 }
 
 }  // namespace
+
+std::string tile_cache_gpu(const char* device_name) { return std::string(device_name) + " kernels 2"; }
 
 std::string tile_cache_path()
 {

@@ -9,6 +9,12 @@
 
 namespace goofy_gpu {
 
+// The GPU name of a cache entry: the device's name and a revision of the image
+// kernels and of what a tile asks of them, raised when either changes so that
+// tiles measured before are not found.  2: 512 x 2 mode 2 stands for a choice
+// by image size; segments and units run across block rows.
+std::string tile_cache_gpu(const char* device_name);
+
 // The cache file in use: the path given to set_tile_cache_path, else
 // $GOOFY_TILE_CACHE, else $XDG_CACHE_HOME/goofy_gb300/tiles.txt, else
 // $HOME/.cache/goofy_gb300/tiles.txt.  "" means no cache.

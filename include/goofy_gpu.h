@@ -201,7 +201,9 @@ int goofy_gpu_set_tile_cache_path(const char* path); /* NULL: back to the enviro
 /* The path in use; copies at most size-1 bytes and a NUL into buf (may be
  * NULL) and returns the full length. */
 size_t goofy_gpu_get_tile_cache_path(char* buf, size_t size);
-/* The GPU name and SM count that key `device`'s entries. */
+/* The GPU name and SM count that key `device`'s entries.  The name ends with
+ * the revision of this library's image kernels: tiles that another revision's
+ * autotuner recorded are not found. */
 int goofy_gpu_device_key(int device, char* name, size_t size, uint32_t* sm_count);
 /* Record / look up one entry directly (path NULL: the path in use).  Need no
  * GPU.  lookup returns GOOFY_ERR_INVALID when there is no valid entry. */
