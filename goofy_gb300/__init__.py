@@ -238,10 +238,10 @@ def _addr(buf):
     if isinstance(buf, int):
         return buf
     if hasattr(buf, "ctypes"):  # numpy
-        try:  # 0.25 us where buf.ctypes.data takes 1.5; needs a writable, C-contiguous array that is not empty
+        try:  # 0.25 us where buf.ctypes.data takes 1.5; needs the buffer of a writable, C-contiguous array
             return ctypes.addressof(_CHAR_AT(buf))
         except (TypeError, ValueError, BufferError):
-            return buf.__array_interface__["data"][0]
+            return buf.ctypes.data
     if isinstance(buf, bytearray):
         return ctypes.addressof((ctypes.c_char * len(buf)).from_buffer(buf))
     if hasattr(buf, "data_ptr"):  # torch tensor
