@@ -241,7 +241,8 @@ def _addr(buf):
         try:  # 0.25 us where buf.ctypes.data takes 1.5; needs the buffer of a writable, C-contiguous array
             return ctypes.addressof(_CHAR_AT(buf))
         except (TypeError, ValueError, BufferError):
-            return buf.ctypes.data
+            info = getattr(buf, "__array_interface__", None)  # read-only arrays and others
+            return info["data"][0] if info else buf.ctypes.data
     if isinstance(buf, bytearray):
         return ctypes.addressof((ctypes.c_char * len(buf)).from_buffer(buf))
     if hasattr(buf, "data_ptr"):  # torch tensor
