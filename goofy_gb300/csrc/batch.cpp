@@ -27,6 +27,7 @@
 #include "../../include/goofy_gpu.h"
 #include "batch.h"
 #include "host_util.h"
+#include "kernels.h"
 
 using goofy_gpu::BatchImage;
 using goofy_gpu::BatchTile;
@@ -70,7 +71,7 @@ constexpr uint32_t kParamLaunches = 2;
 
 namespace {
 
-constexpr uint64_t kResidentWarps = 152 * 32;
+constexpr uint64_t kResidentWarps = goofy_gpu::kSms * 32;
 
 // Checks one image and fills its descriptor (all zero for an empty image).
 int check_image(const goofy_gpu_image& im, BatchImage* out)

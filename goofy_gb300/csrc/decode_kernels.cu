@@ -23,6 +23,7 @@
 #include "decode.h"
 #include "device_io.cuh"
 #include "error_reduce.cuh"
+#include "kernels.h"
 #include "pdl.cuh"
 
 namespace goofy_gpu {
@@ -35,7 +36,7 @@ constexpr uint32_t kDecodeThreads = 256;
 // kernel before it drains (us, inputs of 400 MB in all, BC1: 256^2 1.66 / 1.38,
 // 1024^2 2.7 / 2.4, 2048^2 3.75 / 3.55, 3840x2160 6.1 / 6.0); a larger one's later
 // CTAs start too late for that and would only wait longer (1384x3800 5.05 / 5.2).
-constexpr uint32_t kDecodeWave = 152 * 8;
+constexpr uint32_t kDecodeWave = kSms * 8;
 
 // N blocks a thread, 32 apart, so each store of a warp writes 512 contiguous
 // bytes of a pixel row.

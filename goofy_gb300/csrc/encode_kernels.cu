@@ -244,7 +244,7 @@ static cudaError_t launch_access(const uint8_t* src, size_t stride, uint8_t* dst
 cudaError_t launch_image(int codec, const uint8_t* src, size_t stride, uint8_t* dst, uint32_t width,
                          uint32_t height, Tile tile, SrcAccess access, cudaStream_t stream, uint8_t* dst2, bool host_rows)
 {
-    if (!tile_valid(tile)) return cudaErrorInvalidValue;
+    if (!tile_valid(tile) || (host_rows && tile.persistent == 2)) return cudaErrorInvalidValue;
     if (codec != kBC1 && codec != kETC1S && (codec != kBoth || !dst2)) return cudaErrorInvalidValue;
     const uint32_t bw = width / 4, bh = height / 4;
     if (bw == 0 || bh == 0) return cudaSuccess;
@@ -292,9 +292,14 @@ cudaError_t launch_image(int codec, const uint8_t* src, size_t stride, uint8_t* 
         // each row takes four loads; the other codecs' longer blocks do not, and from 1.7 waves on take the pipeline,
         // whose copies run ahead of the codec.  One big CTA a SM leaves SMs idle in its last round on images of few
         // units, and its one copy queue is slow on short rows.
-        constexpr uint32_t kSms = 152, kTinyBlocks = 20000, kTinyRow = 32, kBigBlocks = 600000, kBigRow = 256;
+        constexpr uint32_t kTinyBlocks = 20000, kTinyRow = 32, kBigBlocks = 600000, kBigRow = 256;
         const bool word = access == SrcAccess::kWord4;
-        // blocks resident at 128x1 and 128x2, by the kernels' registers
+        // One block a thread up to grid1, two (where it can be) up to grid2.  With 16-byte rows these are the blocks
+        // resident at 128x1 and 128x2, by the kernels' registers.  Word-aligned kernels take more (BC1 34, ETC1s 53 at
+        // 128x1: waves of 233,472 and 175,104 blocks; both 73 at 128x2: 233,472), but a little past a wave the next
+        // choice is still slower, in L2 / from HBM: BC1 1940x1944 (235,710) 3.6 / 4.0 against 4.2 / 4.5, 2180^2
+        // (297,025) 4.2 / 4.6 against 4.4 / 4.7, from 2228^2 (310,249) on alike; ETC1s 1760x1756 (193,160) 3.9 / 4.4
+        // against 4.6 / 4.8; both 2048^2 4.9 / 6.45 against 5.9 / 6.5.
         const uint32_t grid1 = kSms * 128 * (codec == kBC1 ? 16 : !word ? 12 : codec == kETC1S ? 10 : 9);
         const uint32_t grid2 = kSms * 256 * (word && codec == kETC1S ? 8 : 7);
         const uint32_t blocks = bw * bh;
@@ -307,7 +312,7 @@ cudaError_t launch_image(int codec, const uint8_t* src, size_t stride, uint8_t* 
         }
         const bool two = blocks > grid1 && (word || (codec != kBC1 && blocks <= grid2));
         tile = Tile{128, two ? 2u : 1u, 0};
-        if (!host_rows) rows = Rows::kAhead;
+        rows = Rows::kAhead;
     } else if (tile.persistent == 0 && !host_rows) {
         // A grid asked for by its shape has its rows prefetched as well, without / with, us, in L2 and from HBM:
         //   128x1 BC1    2048^2 3.9 / 3.5, 4.7 / 3.8    4096^2 12.0 / 10.25, 12.1 / 10.9    6000x4000 16.1 / 18.0
@@ -320,7 +325,7 @@ cudaError_t launch_image(int codec, const uint8_t* src, size_t stride, uint8_t* 
         // 3072^2 9.9 / 9.6; 1024^2 both 4.6 / 3.05).
         const uint32_t blocks = bw * bh;
         const bool word = access == SrcAccess::kWord4, fewer = tile.bpt == 2 && codec != kBC1;
-        const uint32_t wave = 152u * 2u * tile.threads * (tile.threads == 128 ? 7u : tile.threads == 256 ? 3u : 1u);
+        const uint32_t wave = kSms * 2u * tile.threads * (tile.threads == 128 ? 7u : tile.threads == 256 ? 3u : 1u);
         if (fewer && (word || tile.threads > 128) ? blocks <= wave : !word && blocks <= 1250000u) rows = Rows::kAhead;
     }
     if (codec == kBC1) return launch_access<kBC1>(src, stride, dst, nullptr, bw, bh, tile, access, rows, stream);

@@ -8,6 +8,10 @@
 
 namespace goofy_gpu {
 
+// SMs of a GB300.  The launch rules by size are lines measured there, so they
+// take it as a constant; grids that must be resident ask the device.
+constexpr uint32_t kSms = 152;
+
 struct Tile {
     uint32_t threads;     // threads per CTA: 128, 256 or 512
     uint32_t bpt;         // 4x4 blocks per thread and segment: 1, 2 or 4 (1 or 2 when persistent)
@@ -34,7 +38,7 @@ enum class SrcAccess : int {
 // codec kBoth (block_codec.cuh) one pass writes the BC1 blocks to `dst` and
 // the ETC1s blocks to `dst2` (shapes: 1 or 2 blocks a thread; a resident
 // grid with prefetch runs as the plain grid).  `host_rows`: the rows are in
-// host memory (a grid's tile).
+// host memory (a grid's tile: the pipeline's copies take device memory only).
 cudaError_t launch_image(int codec, const uint8_t* src, size_t stride, uint8_t* dst, uint32_t width,
                          uint32_t height, Tile tile, SrcAccess access, cudaStream_t stream, uint8_t* dst2 = nullptr,
                          bool host_rows = false);

@@ -142,9 +142,10 @@ typedef struct goofy_gpu_tile {
                                  *    shared-memory ring with bulk async copies (1, 2 blocks per
                                  *    thread).  Images of under 20,000 blocks or 32 blocks a row run
                                  *    shape 0.  512 x 2 leaves the choice to the image: shape 0 up
-                                 *    to 400,000 blocks (BC1 900,000; word-aligned 311,296 and
-                                 *    600,000), then 128 x 1 here, 512 x 2 for large images;
-                                 *    word-aligned sources run 128 x 1 and 512 x 2 only */
+                                 *    to 400,000 blocks (BC1 900,000; word-aligned rows BC1
+                                 *    600,000, ETC1s 311,296, both codecs in one pass 272,384),
+                                 *    then 128 x 1 here, 512 x 2 for large images; word-aligned
+                                 *    sources run 128 x 1 and 512 x 2 only */
 } goofy_gpu_tile;
 
 /* Get / set the tile the image kernels launch with, per codec
@@ -249,10 +250,12 @@ int goofy_gpu_decode_device(int codec, void* rgba, uint32_t rgba_stride, const v
  * differences, [4] the unsupported-block count, [5] the sum of squared
  * luminosity differences in hundredths, (21 d2 + 72 d1 + 7 d0)^2 with dk the
  * difference of byte k -- the harness's 0.21 R + 0.72 G + 0.07 B of a pixel
- * read as a little-endian u32, exact in integers.  Asynchronous.  Large images
- * are read by the bulk-copy pipeline: the sums miss blocks if one of its
- * bounded waits gave up, which goofy_gpu_pipeline_timeouts counts (the
- * synchronous calls below return GOOFY_ERR_TIMEOUT then). */
+ * read as a little-endian u32, exact in integers.  Asynchronous.  `src` is
+ * device memory; of images of a million blocks and more it is read by bulk
+ * copies, of word-aligned rows in whole 16-byte granules (up to 12 bytes before
+ * and after the rows, of which nothing is used), and the sums miss blocks if one
+ * of the pipeline's bounded waits gave up, which goofy_gpu_pipeline_timeouts
+ * counts (the synchronous calls below return GOOFY_ERR_TIMEOUT then). */
 int goofy_gpu_block_error_device(int codec, const void* blocks, const void* src, uint32_t width, uint32_t height,
                                  uint32_t stride, uint64_t* d_sums, void* stream);
 
