@@ -14,8 +14,8 @@
 // Up to about two thousand images, the descriptors are the kernel's parameter
 // instead (encode_batch_params): no upload and no counter to zero ahead of
 // the kernel, units sized to the work.  A call (us), uploaded / as parameter
-// (both before the prefetches below) / now: 24 tiles of 128x128 12.3 / 2.8 / 2.8,
-// a 2048^2 mip chain 12 / 4 / 4, the first 20 textures of the mixed batch 19.2 / 9.2
+// (both before the prefetches below) / now: 24 tiles of 128x128 12.3 / 3.1 / 3.1
+// (from Python: the host's time), a 2048^2 mip chain 12 / 4 / 4, the first 20 textures of the mixed batch 19.2 / 9.2
 // / 7.0, 100 53.2 / 40.3 / 37.4 (floor 35.5 at 4.5 B/px of measured HBM), 380 (993
 // images) 148 / 137 / 128 (134), 600 (two launches) 201 / 195 / 182.  Each further
 // launch drains the GPU once, about 4 us: with 1000 textures (three launches,

@@ -10,8 +10,8 @@
 // shared between calls, and nothing read from the calling thread's memory
 // after the call returns.  Inputs and outputs are the caller's device buffers.
 // (With the tables written into a device array by a first kernel, 24 tiles of
-// 128x128 took 12.3 us a call; the one launch takes 2.8 us, the host's cost
-// of making it.)
+// 128x128 took 12.3 us a call from Python; the one launch takes 3.1 us, the
+// host's cost of making it.)
 #include <cuda_runtime.h>
 
 #include <cstdio>

@@ -127,9 +127,9 @@ __host__ __device__ constexpr uint32_t l2_prefetch_tiles(const TmaLayout& l)
 // groups a word apart, so no two share a bank.  The codec gives the same block
 // but for the order of its indices (swap_columns in block_codec.cuh).
 // Measured against column order (400 MB of inputs): 4096^2 BC1 13.2 -> 12.2,
-// ETC1s 14.1 -> 13.9 us; 1996x1532 4.4 -> 4.1 and 5.0 -> 4.6.  Four addresses
-// a block plus uniform row offsets: added the other way round (a row's base
-// plus the column) the sixteen sums cost more than the conflicts at 2376x2628.
+// ETC1s 14.1 -> 13.9 us.  Four addresses a block plus uniform row offsets:
+// added the other way round (a row's base plus the column) the sixteen sums
+// cost more than the conflicts at 2376x2628.
 template <int BPT, bool WORD, bool XOR_COLUMNS>
 __device__ __forceinline__ void load_stage(const uint8_t* buf, uint32_t row_bytes, uint32_t warp, uint32_t lane,
                                            uint32_t nb, uint32_t bx0, uint32_t bw, uint32_t bw_magic,
