@@ -258,7 +258,10 @@ cudaError_t launch_block_error(int codec, const uint8_t* blocks, const uint8_t* 
     //                    launches back to back              synchronous calls from Python
     //   1024^2          3.1 / 3.2      4.0 / 3.75         13.4 / 13.7    14.0 / 14.3
     //   2048^2          5.15 / 5.1     5.75 / 5.75        15.5 / 16.5    16.4 / 17.75
+    //   2816^2          7.7 / 7.55     8.0 / 8.8
+    //   3072^2          8.8 / 7.9      9.05 / 8.7         19.4 / 19.5    19.9 / 20.5
     //   3300^2          9.7 / 9.2      9.75 / 10.0        20.2 / 20.9    20.4 / 22.2
+    //   3800^2         12.1 / 11.0    12.1 / 11.5
     //   4096^2         13.1 / 12.0    13.2 / 12.9         23.8 / 24.3    24.0 / 25.15
     //   6000x4000      17.75 / 16.4   17.8 / 16.9         28.1 / 29.05   28.5 / 29.7
     //   8192^2         43.2 / 40.0    44.2 / 42.6         54.0 / 52.6    55.0 / 55.5
@@ -266,7 +269,7 @@ cudaError_t launch_block_error(int codec, const uint8_t* blocks, const uint8_t* 
     //   512x32768      13.1 / 12.6    13.2 / 13.8         23.8 / 24.8    23.85 / 25.3
     // word-aligned 4096^2 13.2 / 14.8, 15.0 / 15.0; 6000x4000 18.3 / 19.8, 19.7 / 20.0; 8192^2 49.0 / 46.8.  ETC1s alike.
     const bool late = result.host || !vec16;
-    if (nblk >= (late ? 2500000u : 1000000u) && bw >= 256)
+    if (nblk >= (late ? 2500000u : 580000u) && bw >= 256)
         return launch_error_tma(codec, blocks, src, width, height, stride, vec16, sums, result, stream);
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);

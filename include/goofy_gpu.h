@@ -251,7 +251,7 @@ int goofy_gpu_decode_device(int codec, void* rgba, uint32_t rgba_stride, const v
  * luminosity differences in hundredths, (21 d2 + 72 d1 + 7 d0)^2 with dk the
  * difference of byte k -- the harness's 0.21 R + 0.72 G + 0.07 B of a pixel
  * read as a little-endian u32, exact in integers.  Asynchronous.  `src` is
- * device memory; of images of a million blocks and more it is read by bulk
+ * device memory; of images of 580,000 blocks and more it is read by bulk
  * copies, of word-aligned rows in whole 16-byte granules (up to 12 bytes before
  * and after the rows, of which nothing is used), and the sums miss blocks if one
  * of the pipeline's bounded waits gave up, which goofy_gpu_pipeline_timeouts
